@@ -31,6 +31,7 @@
 // inside the same launch by the last CTA of the (batch, head, row group) to arrive
 // (merge_splits_in_kernel), or exported for the multi-GPU all-gather (merge_kernel runs after it).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -38,12 +39,67 @@
 
 #include "attn_fused_kernel.cuh"
 #include "attn_tc5_kernel.cuh"
-#include "attn_prefill_kernel.cuh"
 
 #ifndef NOMOS_DS512
 #define NOMOS_DS512 4
 #endif
 namespace nomos {
+
+namespace fused {
+
+// Merge G partial triples per row.  partials [G][rows][hd+2] = (o.., m, l); m in log2
+// units when nat == 0 (in-library split partials), natural-log units when nat == 1.
+// One CTA per row: the weights 2^(m_i - m*) are computed once into shared memory.
+__global__ void __launch_bounds__(128) merge_kernel(const float *partials, int G, int rows, int hd, void *out, int out_type,
+                                                     int nat, float *partial_out) {
+    __shared__ float wgt[MERGE_MAX_G];
+    __shared__ float red[8];
+    pdl_wait();                           // no-op unless launched as a programmatic dependent
+    pdl_launch_dependents();              // a following attention grid may start streaming its cache now
+    const int row = blockIdx.x, tid = threadIdx.x;
+    const float unit = nat ? LOG2E : 1.0f;
+    const size_t rstride = (size_t)rows * (hd + 2);
+    const float *base = partials + (size_t)row * (hd + 2);
+    float mloc = -CUDART_INF_F;
+    for (int i = tid; i < G; i += 128) {
+        const float li = base[i * rstride + hd + 1];
+        const float mi = base[i * rstride + hd] * unit;
+        wgt[i] = li > 0.0f ? mi : -CUDART_INF_F;
+        mloc = fmaxf(mloc, wgt[i]);
+    }
+    mloc = warp_max(mloc);
+    if ((tid & 31) == 0) red[tid >> 5] = mloc;
+    __syncthreads();
+    const float mstar = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    float lloc = 0.0f;
+    for (int i = tid; i < G; i += 128) {
+        const float w = wgt[i] == -CUDART_INF_F ? 0.0f : ex2f(wgt[i] - mstar);
+        lloc += w * base[i * rstride + hd + 1];
+        wgt[i] = w;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lloc += __shfl_xor_sync(0xffffffffu, lloc, o);
+    if ((tid & 31) == 0) red[4 + (tid >> 5)] = lloc;
+    __syncthreads();
+    const float lstar = red[4] + red[5] + red[6] + red[7];
+    for (int d = tid; d < hd; d += 128) {
+        float o = 0.0f;
+        for (int i = 0; i < G; ++i) o = fmaf(wgt[i], base[i * rstride + d], o);
+        if (partial_out) {
+            partial_out[(size_t)row * (hd + 2) + d] = o;
+        } else {
+            const float v = lstar > 0.0f ? o / lstar : 0.0f;
+            if (out_type == ET_BF16) reinterpret_cast<__nv_bfloat16 *>(out)[(size_t)row * hd + d] = __float2bfloat16_rn(v);
+            else reinterpret_cast<float *>(out)[(size_t)row * hd + d] = v;
+        }
+    }
+    if (partial_out && tid == 0) {
+        partial_out[(size_t)row * (hd + 2) + hd] = lstar > 0.0f ? mstar * LN2 : 0.0f;   // exported m: natural log
+        partial_out[(size_t)row * (hd + 2) + hd + 1] = lstar;
+    }
+}
+
+}  // namespace fused
 
 using namespace fused;
 
@@ -690,79 +746,56 @@ static int dispatch_mma(cudaStream_t st, const AttnArgs &a, bool q, long *ws) {
     }
 }
 
+// ------------------------------------------------------------------ query-major prefill (attn_prefill_kernel.cuh)
+// Estimated time of a call as row groups of the mma.sync kernel against the query-major kernel, in us.  Row groups cost per
+// (group, KV head, key); the query-major kernel per 64-key step of a CTA, with one CTA per SM and no split of the keys, so
+// few query rows against a long cache leave the chip idle.  Constants from launches back to back on one box, 512 / 2048 /
+// 16384 keys x 13 to 256 rows (row groups / query-major, us): 32q/16kv x 256 int8, bf16 queries, 2048 keys: 13 rows 21 / 58,
+// 48 rows 54 / 57, 64 rows 53 / 57, 96 rows 78 / 58, 256 rows 184 / 57; 512 keys: 13 rows 13 / 21, 256 rows 74 / 22;
+// 32q/4kv x 512 block-32, 2048 keys: 64 rows 114 / 132, 96 rows 169 / 132, 256 rows 393 / 134.
+static bool prefers_row_groups(const AttnArgs &a) {
+    const bool b32 = a.kv_fmt == KV_I4B32, f32 = a.q_type == ET_F32;
+    const double keys = a.window > 0 ? std::min<long>(a.klen, (long)a.window + a.S - 1) : a.klen;
+    const int rows = a.S * a.kvg, hd = a.l_hd;
+    const double per_group = hd == 128 ? (a.kv_fmt == KV_I8 ? 70e-6 : 117e-6) : hd == 256 ? 76e-6 : 168e-6;    // us per (group, head, key)
+    const double t_groups = 8.0 + per_group * ((rows + (hd == 128 ? 23 : 7)) / (hd == 128 ? 24 : 8)) * keys * a.nkv * a.batch;
+    const int nq = hd == 128 ? 2 : 1, dsplit = hd == 512 ? 2 : 1, tiles_q = (rows + 127) / 128;
+    const bool both = nq == 2 && tiles_q > 1;
+    double step;                                       // us per 64 keys
+    if (hd == 128) step = b32 ? (f32 ? (both ? 3.1 : 2.4) : (both ? 2.1 : 1.4)) : (f32 ? (both ? 1.8 : 1.1) : (both ? 1.45 : 1.05));
+    else if (hd == 256) step = b32 ? (f32 ? 3.0 : 2.2) : (f32 ? 2.0 : 1.5);
+    else step = b32 ? 3.8 : 2.1;
+    const double ctas = (double)((tiles_q + nq - 1) / nq) * a.nkv * dsplit * a.batch, span = 128.0 * nq / a.kvg;
+    const double longest = a.window > 0 ? std::min<double>(a.klen, a.window + span) : a.klen;
+    const double mean = a.window > 0 ? longest : std::max(64.0, a.klen - 0.5 * a.S);
+    const double waves = std::ceil(ctas / device_info().sm_count);
+    const double t_query = 11.0 * std::min(waves, 2.0) + step / 64.0 * std::max(longest, std::max(ctas * mean / device_info().sm_count, a.window > 0 ? waves * mean : 0.0));
+    return t_groups < 1.2 * t_query;                  // (the estimates are good to about a fifth)
+}
+
+// More query rows per KV head than the decode / verify kernels serve in one CTA (24), no fused append and no partial
+// export.  fp32 queries of 512-wide heads (two fp16 limbs of a query tile do not fit beside the operand ring) run as row
+// groups of the mma.sync kernel, and so do the formats and widths below that these suit better; int8 / head_dim 128, and
+// prefix ranges that only this kernel expresses, always come here.
+static bool prefill_eligible(const AttnArgs &a) {
+    if (a.no_tma || a.no_tcgen05 || a.block_table != nullptr) return false;
+    if (a.new_k != nullptr || a.partial_out != nullptr || a.out == nullptr || a.peer_world > 1) return false;
+    if (!a.d0_set && a.S * a.kvg <= 24) return false;
+    if (a.kvg != 1 && a.kvg != 2 && a.kvg != 4 && a.kvg != 8) return false;
+    if (a.l_hd == 512 && a.q_type != ET_BF16) return false;
+    if ((a.kv_fmt != KV_I8 || a.l_hd != 128) && !a.tcgen05_always && prefers_row_groups(a)) return false;
+    const auto al16 = [](const void *x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
+    if (!al16(a.k_cache) || !al16(a.v_cache) || !al16(a.q) || !al16(a.out) || a.cache_hd % (a.kv_fmt == KV_I8 ? 16 : 32) != 0) return false;
+    if (a.q_batch_stride % 8 != 0 || a.out_batch_stride % 8 != 0 || a.scale_batch_stride % 4 != 0) return false;
+    if (a.batch > 1 && a.kv_batch_stride % 16 != 0) return false;
+    return true;
+}
+
 // Calls both kernels can serve, decode shapes (up to 8 query rows per KV head).  Measured on B200 with both on
 // one box: the tcgen05 kernel streams faster (batch 8 x 131072 keys 619 vs 641 us, 524288 keys 325 vs 346 us:
 // about 7.0 against 6.6 TB/s), the mma.sync kernel has about 2 us less fixed cost per call (one CTA per SM, half
 // as many partials to merge).  The crossing point moved from about 240 MB to about 330 MB of cache when the
 // mma.sync kernel's tile copies became evict-first in L2; the table the threshold is read from is at prefers_mma().
-// ------------------------------------------------------------------ query-major prefill (attn_prefill_kernel.cuh)
-// int8 KV, head_dim 128, more query rows per KV head than the decode / verify kernels serve in one CTA (24), a
-// window that does not wrap the ring, no fused append and no partial export.  Everything else -- int4 caches, wider
-// heads, wrapped rings -- runs as row groups of the mma.sync kernel (also without any S x key_len scratch).
-static bool prefill_eligible(const AttnArgs &a) {
-    if (a.kv_fmt != KV_I8 || a.l_hd != 128 || a.no_tma || a.no_tcgen05 || a.block_table != nullptr) return false;
-    if (a.new_k != nullptr || a.partial_out != nullptr || a.out == nullptr || a.peer_world > 1) return false;
-    if (!a.d0_set && a.S * a.kvg <= 24) return false;
-    if (a.kvg != 1 && a.kvg != 2 && a.kvg != 4 && a.kvg != 8) return false;
-    if ((long)(a.win_start % a.cache_cap) + a.klen > a.cache_cap) return false;
-    if (encode_tiled_fn() == nullptr) return false;
-    const auto al16 = [](const void *x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
-    if (!al16(a.k_cache) || !al16(a.v_cache) || !al16(a.q) || !al16(a.out) || a.cache_hd % 16 != 0) return false;
-    if (a.q_batch_stride % 8 != 0 || a.out_batch_stride % 8 != 0 || a.scale_batch_stride % 4 != 0) return false;
-    if (a.batch > 1 && a.kv_batch_stride % 16 != 0) return false;
-    if ((long)a.nkv * a.cache_cap >= (1l << 31)) return false;
-    return true;
-}
-
-static int launch_prefill(cudaStream_t st, const AttnArgs &a) {
-    static bool attr_set[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!attr_set[dev]) {
-        cudaFuncSetAttribute(pf::attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pf::SMEM_BYTES);
-        attr_set[dev] = true;
-    }
-    pf::PMaps tm;
-    const int rows = a.nkv * a.cache_cap;
-    const MapKey mk{a.k_cache, 0, 128, a.cache_hd, rows, a.batch, pf::KT, a.kv_batch_stride};
-    const MapKey mv{a.v_cache, 0, 128, a.cache_hd, rows, a.batch, pf::KT, a.kv_batch_stride};
-    if (!encode_plane(mk, &tm.k) || !encode_plane(mv, &tm.v)) return 1;
-    pf::PParams p;
-    std::memset(&p, 0, sizeof(p));
-    p.q = static_cast<const uint8_t *>(a.q);
-    p.out = static_cast<uint8_t *>(a.out);
-    p.k_scales = static_cast<const float *>(a.k_scales);
-    p.v_scales = static_cast<const float *>(a.v_scales);
-    p.q_type = a.q_type; p.out_type = a.out_type;
-    p.S = a.S; p.nh = a.nh; p.nkv = a.nkv; p.kvg = a.kvg; p.cache_cap = a.cache_cap;
-    p.row0 = a.win_start % a.cache_cap;
-    p.key_len = a.klen;
-    p.d0 = a.d0_set ? a.d0 : a.klen - a.S;
-    p.window = a.window;
-    p.pos_per_cta = pf::MR / a.kvg;
-    p.q_blocks = (a.S + p.pos_per_cta - 1) / p.pos_per_cta;
-    p.q_scale = a.softmax_scale * LOG2E;
-    p.q_batch_stride = a.q_batch_stride; p.out_batch_stride = a.out_batch_stride; p.scale_batch_stride = a.scale_batch_stride;
-    p.scales_vec = ((reinterpret_cast<uintptr_t>(a.k_scales) | reinterpret_cast<uintptr_t>(a.v_scales)) % 16 == 0 && a.cache_cap % 4 == 0 &&
-                    p.row0 % 4 == 0 && a.scale_batch_stride % 16 == 0) ? 1 : 0;
-    p.fault = fault_word();
-    if (p.fault == nullptr) { set_error("attn_prefill: device fault word unavailable"); return NOMOS_ECUDA; }
-    if (p.q_blocks > 65535 * 32 || a.batch > 65535) { set_error("attn_prefill: too many query blocks"); return NOMOS_EUNSUPPORTED; }
-    cudaLaunchAttribute pdl[1];
-    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pdl[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.q_blocks, a.nkv, a.batch);
-    cfg.blockDim = dim3(pf::NTHREADS);
-    cfg.dynamicSmemBytes = pf::SMEM_BYTES;
-    cfg.stream = st;
-    cfg.attrs = pdl; cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, pf::attn_prefill_kernel, p, tm);
-    if (e != cudaSuccess) { set_error("attn_prefill launch: %s", cudaGetErrorString(e)); return NOMOS_ECUDA; }
-    return NOMOS_OK;
-}
-
 static bool prefers_mma(const AttnArgs &a) {
     if (a.tcgen05_always || a.block_table != nullptr || a.S * a.kvg > 8) return false;
     const int keys = a.window > 0 ? std::min(a.klen, a.window + a.S - 1) : a.klen;
@@ -773,10 +806,7 @@ static bool prefers_mma(const AttnArgs &a) {
 }
 
 static int dispatch(cudaStream_t st, const AttnArgs &a, bool q, long *ws) {
-    if (!q && prefill_eligible(a)) {
-        const int rc = launch_prefill(st, a);
-        if (rc != 1) return rc;                    // 1: the tensor maps could not be encoded, use the other kernels
-    }
+    if (!q && prefill_eligible(a)) return launch_attn_prefill(st, a, fault_word());
     if (a.d0_set) { set_error("this key range needs the prefill kernel (int8 KV, head_dim 128, 16-byte aligned buffers)"); return NOMOS_EUNSUPPORTED; }
     if (!tc5_eligible(a)) return dispatch_mma(st, a, q, ws);
     if (q) {

@@ -1709,58 +1709,7 @@ __global__ void __launch_bounds__(Cfg<FMT, HD, MT, DS, QS>::NW * 32)
     merge_splits_in_kernel<C::NSLOT, HD, NWARP * 32>(p, pipe, b, kvh, rg);
 }
 
-// Merge G partial triples per row.  partials [G][rows][hd+2] = (o.., m, l); m in log2
-// units when nat == 0 (in-library split partials), natural-log units when nat == 1.
-// One CTA per row: the weights 2^(m_i - m*) are computed once into shared memory.
-constexpr int MERGE_MAX_G = 1024;
-__global__ void __launch_bounds__(128) merge_kernel(const float *partials, int G, int rows, int hd, void *out, int out_type,
-                                                     int nat, float *partial_out) {
-    __shared__ float wgt[MERGE_MAX_G];
-    __shared__ float red[8];
-    pdl_wait();                           // no-op unless launched as a programmatic dependent
-    pdl_launch_dependents();              // a following attention grid may start streaming its cache now
-    const int row = blockIdx.x, tid = threadIdx.x;
-    const float unit = nat ? LOG2E : 1.0f;
-    const size_t rstride = (size_t)rows * (hd + 2);
-    const float *base = partials + (size_t)row * (hd + 2);
-    float mloc = -CUDART_INF_F;
-    for (int i = tid; i < G; i += 128) {
-        const float li = base[i * rstride + hd + 1];
-        const float mi = base[i * rstride + hd] * unit;
-        wgt[i] = li > 0.0f ? mi : -CUDART_INF_F;
-        mloc = fmaxf(mloc, wgt[i]);
-    }
-    mloc = warp_max(mloc);
-    if ((tid & 31) == 0) red[tid >> 5] = mloc;
-    __syncthreads();
-    const float mstar = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-    float lloc = 0.0f;
-    for (int i = tid; i < G; i += 128) {
-        const float w = wgt[i] == -CUDART_INF_F ? 0.0f : ex2f(wgt[i] - mstar);
-        lloc += w * base[i * rstride + hd + 1];
-        wgt[i] = w;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lloc += __shfl_xor_sync(0xffffffffu, lloc, o);
-    if ((tid & 31) == 0) red[4 + (tid >> 5)] = lloc;
-    __syncthreads();
-    const float lstar = red[4] + red[5] + red[6] + red[7];
-    for (int d = tid; d < hd; d += 128) {
-        float o = 0.0f;
-        for (int i = 0; i < G; ++i) o = fmaf(wgt[i], base[i * rstride + d], o);
-        if (partial_out) {
-            partial_out[(size_t)row * (hd + 2) + d] = o;
-        } else {
-            const float v = lstar > 0.0f ? o / lstar : 0.0f;
-            if (out_type == ET_BF16) reinterpret_cast<__nv_bfloat16 *>(out)[(size_t)row * hd + d] = __float2bfloat16_rn(v);
-            else reinterpret_cast<float *>(out)[(size_t)row * hd + d] = v;
-        }
-    }
-    if (partial_out && tid == 0) {
-        partial_out[(size_t)row * (hd + 2) + hd] = lstar > 0.0f ? mstar * LN2 : 0.0f;   // exported m: natural log
-        partial_out[(size_t)row * (hd + 2) + hd + 1] = lstar;
-    }
-}
+constexpr int MERGE_MAX_G = 1024;            // most splits the merge kernel takes
 
 }  // namespace fused
 }  // namespace nomos

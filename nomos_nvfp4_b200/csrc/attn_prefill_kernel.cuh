@@ -1,38 +1,34 @@
-// Query-major flash prefill over the int8 KV cache on the fifth-generation tensor cores (tcgen05 + tensor
-// memory), head_dim 128, sm_100a.  The host side (eligibility, tensor maps, launch) is in attn_fused.cu.
+// Query-major flash prefill straight off the packed KV cache on the fifth-generation tensor cores (tcgen05 + tensor
+// memory), sm_100a: int8, int4 and block-32 int4 caches, head dims 128 / 256 / 512.  The host side (eligibility, launch)
+// is in attn_fused.cu.
 //
 // Replaces the reference's square / prefix batched prefill attention
 //   lib/attention_gpu_int8.mojo:804-887 (int8), lib/batched_attn_gpu.mojo:448-666 (fp32 / bf16 twins)
 // which materialise an [nkv, S*kvg, key_len] score matrix in device memory (the reference's own note on the
 // "real fix": lib/engine_prefill.mojo:145; the cap it forces on prompts: pyhost/serve.py:41-64).  Nothing of size
-// S x key_len exists here: a CTA owns 128 query rows and walks the key tiles they may attend.
+// S x key_len exists here: a CTA owns 128 or 256 query rows and walks the key tiles they may attend.
 //
-// One CTA = 128 query rows of ONE KV head: 128 / kvg consecutive query positions x the kvg query heads of the
-// group (position-major, so causal bounds are monotone in the row index), against key tiles of 128 keys.
-//   S[128 rows x 128 keys]  = Qlimb[128 x 128 B] (A, K-major, int8) x K_tile[128 keys x 128 B]^T (B, K-major, int8)
-//                             once per query limb, kind::i8, int32 accumulators S_hi and S_lo in tensor memory.
-//                             B is the K bytes exactly as TMA wrote them; the query is a 16-bit fixed point per row
-//                             (two int8 limbs), so the integer dot product is exact.
-//   O[128 rows x 128 dims] += Plimb[128 x 128 keys] (A, K-major, fp16) x V16[128 keys x 128 dims] (B, MN-major, fp16)
-//                             once per weight limb, kind::f16, one fp32 accumulator in tensor memory across all tiles.
-//                             V16 holds the int8 CODES of V (exact in fp16), converted by four "dequant" warps; the
-//                             softmax weight times the value's row scale is split into fp16 hi + lo, so the weights
-//                             carry 22 bits.  (With single fp16 weights the result sat 0.7e-3 x RMS from exact
-//                             arithmetic at the median and 2e-3 in the tail over a few thousand rows -- the rounding
-//                             of P does not average out against the row's RMS -- which is the accuracy bar itself.)
-// The row scales are applied in fp32 by the softmax threads: the key's to the logit, the value's to the weight.
-// The cache stays int8 in device memory and on the way in: TMA boxes of 128 rows x 128 bytes, one tensor map per
-// plane over this GPU's own memory, no cluster, nothing multicast.
+// A query tile = 128 rows of ONE KV head: 128 / kvg consecutive query positions x the kvg query heads of the group
+// (position-major, so causal bounds are monotone in the row index).  Per key tile of KT keys:
+//   S[128 x KT]  = Q16[128 x HD] (A, shared memory) x K16[KT x HD]^T (B, K-major)           kind::f16, fp32 accumulate
+//   O[128 x DV] += P16[128 x KT] (A, TENSOR memory) x V16[KT x DV] (B, MN-major: [key][dim] as stored)
+// Operands are fp16 and carry all the bits of what they stand for:
+//   Q16  the query row times a power of two of its own (bf16 rows fit one fp16 exactly; fp32 rows take hi + lo, 22 bits)
+//   K16, V16  the cache CODES (exact in fp16), row scales applied in fp32 afterwards; block-32 rows: code x fp16 block
+//        scale is up to 14 bits, split into code x (top 7 bits of the scale) + code x (the other 4), both exact
+//   P16  the softmax weight times the value's row scale as hi + lo (22 bits)
+// The value scale rides in the exponent: with u' = logit + log2(vscale) the weight is w = 2^(u' - m), m a whole-number
+// running reference of u', so w fits fp16 whatever the scale, and the denominator takes w / vscale.
 //
-// Roles (640 threads): warps 0-15 softmax -- query row r = TMEM lane r is shared by four threads, lane r % 32 of warps
-// r / 32 + 4 q, q = 0..3 (all may read that lane quarter), each taking 32 of the tile's 128 keys: four warps per
-// scheduler hide each other's latencies (one warp per scheduler measured 0.16 instructions per cycle, two 0.34), the
-// row maximum crosses the four through shared memory once per tile; warps 16-17 dequant (a thread converts two key rows
-// of the V tile), warp 18 lane 0 TMA producer (+ TMEM allocation), warp 19 lane 0 MMA issuer.  The softmax threads pull
-// S into registers and release it at once, so QK of tile i+1 runs while they work on tile i; O stays in tensor memory across tiles and is rescaled in
-// place only when a row's running maximum moves by more than 2^8 (a handful of times per row).  Every wait is an
-// mbarrier wait with a time limit; a wait that runs out raises the CTA's abort flag and bit 1 of the device fault
-// word, every role leaves its loop, tensor memory is freed and the CTA exits.
+// Roles: per query tile four softmax warps (thread = query row = TMEM lane: S is read 32 columns at a time and the
+// weights go back into the SAME columns, hi and lo, as the A operand of PV); "dequant" warps that fetch cache bytes
+// from global memory one operand slot ahead, widen them and fill a ring of K / V slots in the order the tensor core
+// takes them (rows are addressed one by one: rings may wrap); one MMA warp.  head_dim 128: two query tiles per CTA in
+// turn, one tile's softmax under the other's products; wider heads: one query tile with two S buffers, and at 512 two
+// CTAs per query tile that each own 256 output dims.  O stays in tensor memory; it is rescaled in place only when a
+// row's reference moves, which happens when a chunk exceeds it by more than 2^8 (a handful of times per row).
+// Every wait is an mbarrier wait with a time limit; a wait that runs out raises the CTA's abort flag and bit 1 of the
+// device fault word, every role leaves its loop, tensor memory is freed and the CTA exits.
 #pragma once
 
 #include "attn_tc5_kernel.cuh"
@@ -43,58 +39,79 @@ namespace pf {
 using fused::LOG2E;
 using tc5::wait_or_abort;
 
-constexpr int KT = 128;                       // keys per tile
-constexpr int HD = 128;                       // head dim
-constexpr int MR = 128;                       // query rows per CTA
-constexpr int RAW_TILE = KT * HD;             // int8 tile as TMA writes it (16 KB)
-constexpr int H_TILE = KT * HD * 2;           // fp16 operand tile (32 KB) = two 64-column blocks of 16 KB
-constexpr int H_BLOCK = 16384;
+constexpr int MR = 128;                       // query rows per tile = M of the MMAs
 constexpr float M_INIT = -1.0e30f;
-constexpr float LAZY = 8.0f;                  // base-2 slack before a row's running maximum is moved
+constexpr float LAZY = 8.0f;                  // base-2 slack before a row's running reference is moved
+constexpr float VS_MIN = 1.0e-30f;            // value scales below this count as this (codecs write none)
+constexpr int KT = 64;                        // keys per tile
+constexpr int SMEM_MAX = 232448;              // shared memory a CTA may ask for
 
-constexpr int OFF_RAW = 0;                    // [2 stages][K, V] int8 as TMA writes them
-constexpr int OFF_V16 = 2 * 2 * RAW_TILE;     // 65536: V codes as fp16
-constexpr int OFF_Q8 = OFF_V16 + H_TILE;      // query limbs: high, then low ([128 rows x 128 B] int8 each)
-constexpr int OFF_P16 = OFF_Q8 + 2 * RAW_TILE;   // weight limbs: high, then low (fp16 operand tiles)
-constexpr int OFF_BAR = OFF_P16 + 2 * H_TILE; // 196608
-constexpr int NBAR = 16;
-constexpr int OFF_MISC = OFF_BAR + NBAR * 8;  // tmem base, abort flag
-constexpr int OFF_SC = OFF_MISC + 64;         // [2 stages][K scales | V scales] fp32, 128 each, bulk-copied with the tile
-constexpr int TPR = 4;                        // softmax threads per query row
-constexpr int KPT = KT / TPR;                 // keys of a tile (and dims of Q / O) per softmax thread
-constexpr int NSOFT = TPR * MR;               // softmax threads
-constexpr int W_DEQ = NSOFT / 32;             // first of the two dequant warps; then the TMA producer, then the MMA issuer
-constexpr int W_TMA = W_DEQ + 2, W_MMA = W_DEQ + 3;
-constexpr int OFF_XCH = OFF_SC + 2 * 2 * KT * 4;        // [3][TPR][128 rows] fp32: row maxima by tile parity; region 2: query maxima, then denominators
-constexpr int SMEM_BYTES = 1024 + OFF_XCH + 3 * TPR * 128 * 4;
-constexpr int NTHREADS = NSOFT + 128;
-static_assert(KPT == 32, "a softmax thread moves one 32-column block of tensor memory per limb");
-constexpr int TMEM_COLS = 512;                // S_hi at column 0, S_lo at 128, O at 256
-constexpr int Q_FIX_MAX = fused::Q_FIX_MAX;   // 16-bit fixed-point query, two int8 limbs
-static_assert(OFF_V16 % 1024 == 0 && OFF_Q8 % 1024 == 0 && OFF_P16 % 1024 == 0, "operand tiles sit on swizzle-pattern boundaries");
-static_assert(OFF_SC % 16 == 0, "bulk copies land on 16-byte boundaries");
-static_assert(SMEM_BYTES <= 232448, "shared memory budget of a CTA");
+constexpr int cmin(int a, int b) { return a < b ? a : b; }
+
+template <int HD_, int FMT_, int QL_>
+struct Cfg {
+    static constexpr int HD = HD_, FMT = FMT_, QL = QL_;               // QL: fp16 limbs of the query
+    static constexpr int KL = FMT == KV_I4B32 ? 2 : 1;                 // fp16 limbs of K and V
+    static constexpr int NQ = HD == 128 ? 2 : 1;                       // query tiles per CTA
+    static constexpr int DV = cmin(HD, 256);                           // output dims per CTA
+    static constexpr int DSPLIT = HD / DV;
+    static constexpr int Q_BLOCK = MR * 128;                           // 64 dims of a query tile (one swizzle block column)
+    static constexpr int Q_LIMB = Q_BLOCK * (HD / 64);
+    static constexpr int Q_BYTES = NQ * QL * Q_LIMB;
+    static_assert(Q_BYTES <= 131072, "the query tiles stay resident");
+    static constexpr int BLOCK = KT * 128;                             // 64 dims of KT keys
+    static constexpr int SLOT = 2 * BLOCK;                             // ring slot: KT keys x 128 dims, fp16
+    static constexpr int KS = HD / 128 * KL, VS = DV / 128 * KL;       // slots of a K tile, of a V tile
+    // Per-key constants of tile i are overwritten at tile i + nconst, behind the wait for that tile's first K slot, which
+    // the ring grants only once V of tile i is released (all softmax rows of tile i are then done): ring order
+    // K0 K1 V0 K2 V1 ... makes that (nconst - 2) * (KS + VS) >= slots - 1.
+    static constexpr int nconst(int slots) { return 2 + (slots - 1 + KS + VS - 1) / (KS + VS); }
+    static constexpr int smem(int slots) { return Q_BYTES + slots * SLOT + nconst(slots) * 3 * KT * 4 + (2 * slots + nconst(slots) + 4 * NQ + 2 * NQ + 1) * 8 + 16; }
+    static constexpr int most_slots() { int n = 2 * KL; while (smem(n + KL) <= SMEM_MAX) n += KL; return n; }
+    static constexpr int NSLOT = most_slots(), NCONST = nconst(NSLOT);
+    static_assert(NSLOT >= 2 * KL && NSLOT % KL == 0, "a V unit and the K unit behind it; the limbs of a unit side by side");
+    static constexpr int NSB = 2 * NQ;                                 // S buffers: two per query tile
+    static constexpr int TMEM_O = 0, TMEM_S = 256;
+    static_assert(NQ * DV <= 256 && NSB * KT <= 256, "tensor memory columns");
+    static constexpr int NSW = 8 * NQ;                                 // softmax warps: two per 32 TMEM lanes, 16 rows each
+    // Dequant warps, in teams of two that take the units (KL slots) in turn: what a unit costs a team besides its bytes
+    // (slot wait, address arithmetic, proxy fence, hand-off: about 1500 cycles) overlaps the other teams'.
+    // No more teams than the ring holds units: a slot's next user may not wait for a phase of its barrier whose
+    // predecessor is still pending (products release the slots in order, so with this many none can).
+    static constexpr int TEAMS = cmin(NQ == 2 ? 3 : 5, NSLOT / KL), ND = 2 * TEAMS;
+    static constexpr int W_DEQ = NSW, W_MMA = NSW + ND;
+    static constexpr int NTHREADS = 32 * (NSW + ND + 1);
+    static constexpr int OFF_Q = 0;
+    static constexpr int OFF_RING = Q_BYTES;
+    static constexpr int OFF_CONST = OFF_RING + NSLOT * SLOT;          // [NCONST][3][KT] fp32: logit factor, log2(vscale), 1 / vscale
+    static constexpr int OFF_BAR = OFF_CONST + NCONST * 3 * KT * 4;
+    static constexpr int NBAR = 2 * NSLOT + NCONST + 3 * NSB + 1;
+    static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;
+    static constexpr int SMEM_BYTES = OFF_MISC + 16;                   // (no static shared memory: the dynamic part starts 1024-byte aligned)
+    static_assert(SMEM_BYTES == smem(NSLOT) && SMEM_BYTES <= SMEM_MAX, "shared memory budget of a CTA");
+    // dequant work of a slot: 16-byte pieces of cache bytes
+    static constexpr int CPP = FMT == KV_I8 ? 16 : 32;                 // codes per piece
+    static constexpr int PPR = 128 / CPP;                              // pieces per row of a slot
+    static constexpr int NP = KT * PPR / 64;                           // pieces per thread and slot
+    static constexpr int NBW = HD / 64;                                // block-32: 32-bit words of fp16 scales per row
+};
 
 struct PParams {
     const uint8_t *q;
     uint8_t *out;
-    const float *k_scales, *v_scales;         // fp32 row scales [batch][nkv][cache_cap]
-    int q_type, out_type;
-    int S, nh, nkv, kvg, cache_cap;
-    int row0;                                 // cache slot of key index 0 of the array (win_start; the window does not wrap)
+    const uint8_t *k_cache, *v_cache, *k_scales, *v_scales;
+    int out_type;
+    int batch, S, nh, nkv, kvg, cache_cap;
+    int row_bytes;                            // bytes of a cache row
+    int row0;                                 // ring slot of key index 0 of the array
     int key_len;                              // keys of the array
     int d0;                                   // query row s may attend key indices <= d0 + s (d0 may be negative)
     int window;                               // > 0: and no key index below d0 + s - window + 1
-    int pos_per_cta;                          // 128 / kvg
+    int pos_per_tile;                         // 128 / kvg
     int q_blocks;
-    int scales_vec;                           // 1: a tile's scales start on a 16-byte boundary (vector loads)
     float q_scale;                            // softmax_scale * log2(e)
-    long q_batch_stride, out_batch_stride, scale_batch_stride;
+    long q_batch_stride, out_batch_stride, kv_batch_stride, scale_batch_stride;
     unsigned int *fault;
-};
-
-struct PMaps {
-    CUtensorMap k, v;                         // {row bytes, nkv * cache_cap rows, batch}, box {128 B, 128 rows, 1}, 128B swizzle
 };
 
 // ---------------------------------------------------------------- PTX wrappers
@@ -108,115 +125,176 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// A operand in tensor memory (fp16 pairs in 32-bit columns, lane = row)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // Instruction descriptor for kind::f16: fp32 accumulate, fp16 A and B, M = 128, given N; B may be MN-major.
-__device__ __forceinline__ uint32_t make_idesc_f16(int n, bool b_mn_major) {
+__device__ __forceinline__ constexpr uint32_t make_idesc_f16(int n, bool b_mn_major) {
     return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
-// This warp's 32 TMEM lanes x 32 consecutive 32-bit columns: thread t gets lane t's row.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&r)[32]) {
-    uint32_t u[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
-          "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]),
-          "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]),
-          "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) r[i] = __uint_as_float(u[i]);
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(pred));
+    return pred != 0;
 }
-__device__ __forceinline__ void tmem_ld16i(uint32_t taddr, int (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
+// This warp's 32 TMEM lanes x 32 consecutive 32-bit columns: thread t gets lane t's row.  The caller waits.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n" ::"r"(taddr),
-        "r"(__float_as_uint(r[0])), "r"(__float_as_uint(r[1])), "r"(__float_as_uint(r[2])), "r"(__float_as_uint(r[3])),
-        "r"(__float_as_uint(r[4])), "r"(__float_as_uint(r[5])), "r"(__float_as_uint(r[6])), "r"(__float_as_uint(r[7])),
-        "r"(__float_as_uint(r[8])), "r"(__float_as_uint(r[9])), "r"(__float_as_uint(r[10])), "r"(__float_as_uint(r[11])),
-        "r"(__float_as_uint(r[12])), "r"(__float_as_uint(r[13])), "r"(__float_as_uint(r[14])), "r"(__float_as_uint(r[15])),
-        "r"(__float_as_uint(r[16])), "r"(__float_as_uint(r[17])), "r"(__float_as_uint(r[18])), "r"(__float_as_uint(r[19])),
-        "r"(__float_as_uint(r[20])), "r"(__float_as_uint(r[21])), "r"(__float_as_uint(r[22])), "r"(__float_as_uint(r[23])),
-        "r"(__float_as_uint(r[24])), "r"(__float_as_uint(r[25])), "r"(__float_as_uint(r[26])), "r"(__float_as_uint(r[27])),
-        "r"(__float_as_uint(r[28])), "r"(__float_as_uint(r[29])), "r"(__float_as_uint(r[30])), "r"(__float_as_uint(r[31]))
-        : "memory");
+// 16 lanes x 8 n columns, spread over the warp like an MMA accumulator: registers 4 e + 2 r + {0, 1} of a thread are
+// columns 8 e + 2 (lane % 4) + {0, 1} of row 8 r + lane / 4.  The caller waits.
+__device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st_frag32(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// The same rows, packed pairs: register 2 e + r is column 4 e + lane % 4 of row 8 r + lane / 4.
+__device__ __forceinline__ void tmem_st_pairs32(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-// Byte offset of 16-byte chunk `chunk` (0..15) of row `row` in an fp16 operand tile: two blocks of 64 columns,
-// each [128 rows x 128 bytes] in the 128-byte swizzle pattern (8-row groups 1024 bytes apart).
-__device__ __forceinline__ int h_off(int row, int chunk) {
-    return (chunk >> 3) * H_BLOCK + (row >> 3) * 1024 + (row & 7) * 128 + (((chunk & 7) ^ (row & 7)) << 4);
+// two floats per instruction
+struct __align__(8) F2 { float x, y; };
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("{\n.reg .b64 ra, rb, rc, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmov.b64 rc, {%6, %7};\n"
+        "fma.rn.f32x2 rd, ra, rb, rc;\nmov.b64 {%0, %1}, rd;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 d;
+    asm("{\n.reg .b64 ra, rb, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmul.rn.f32x2 rd, ra, rb;\nmov.b64 {%0, %1}, rd;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 d;
+    asm("{\n.reg .b64 ra, rb, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nadd.rn.f32x2 rd, ra, rb;\nmov.b64 {%0, %1}, rd;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float pow2i(int e) {                        // 2^e, e clamped to the normal range
+    return __int_as_float((max(-126, min(127, e)) + 127) << 23);
+}
+
+// Byte offset of 16-byte chunk `chunk` (8 dims) of row `row` in an operand tile of fp16 rows: blocks of 64 dims, each
+// [rows x 128 bytes] in the 128-byte swizzle pattern (8-row groups 1024 bytes apart).
+__device__ __forceinline__ int op_off(int row, int chunk, int block_bytes) {
+    return (chunk >> 3) * block_bytes + (row >> 3) * 1024 + (row & 7) * 128 + (((chunk & 7) ^ (row & 7)) << 4);
 }
 // Four int8 codes -> the same four integers as fp16.  The bytes become 1024 + (code + 128) as fp16 bit patterns
 // (0x6400 | u8); subtracting 1152 is exact.
 __device__ __forceinline__ void cvt4(uint32_t codes, uint32_t &lo, uint32_t &hi) {
     const uint32_t u = codes ^ 0x80808080u;
-    const uint32_t p0 = prmt(u, 0x64646464u, 0x4140u);       // bytes (u0, 0x64, u1, 0x64) -> halves 1024+u0, 1024+u1
-    const uint32_t p1 = prmt(u, 0x64646464u, 0x4342u);
-    const __half2 bias = __float2half2_rn(1152.0f);
-    const __half2 c0 = __hsub2(*reinterpret_cast<const __half2 *>(&p0), bias);
-    const __half2 c1 = __hsub2(*reinterpret_cast<const __half2 *>(&p1), bias);
-    lo = *reinterpret_cast<const uint32_t *>(&c0);
-    hi = *reinterpret_cast<const uint32_t *>(&c1);
+    lo = hsub2_u32(prmt(u, 0x64646464u, 0x4140u), 0x64806480u);
+    hi = hsub2_u32(prmt(u, 0x64646464u, 0x4342u), 0x64806480u);
+}
+// Eight int4 codes (element 2j in the low nibble of byte j) -> fp16 pairs (0,1) (2,3) (4,5) (6,7).  A nibble becomes
+// 1024 + (code + 8) as an fp16 bit pattern; subtracting 1032 is exact.
+__device__ __forceinline__ void cvt8_i4(uint32_t w, uint32_t (&h)[4]) {
+    uint32_t e[4];                                                     // elements (k, k + 4)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e[k] = hsub2_u32(lop3_and_xor(w >> (4 * k), 0x000f000fu, 0x64086408u), 0x64086408u);
+    h[0] = prmt(e[0], e[1], 0x5410u); h[1] = prmt(e[2], e[3], 0x5410u);
+    h[2] = prmt(e[0], e[1], 0x7632u); h[3] = prmt(e[2], e[3], 0x7632u);
+}
+__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// Block-32 rows: power of two that takes the row's largest block scale to [2^11, 2^12) (times any code it stays below
+// the fp16 maximum, and the low limb of a block 2^-10 of the largest still has all its bits).
+template <int NBW>
+__device__ __forceinline__ int b32_shift(const uint32_t (&w)[NBW]) {
+    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < NBW; ++i) mx = max(mx, max(w[i] & 0x7fffu, (w[i] >> 16) & 0x7fffu));
+    return 26 - max(1, (int)(mx >> 10));
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1) attn_prefill_kernel(const __grid_constant__ PParams p, const __grid_constant__ PMaps tm) {
+template <int HD, int FMT, int QL>
+__global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_kernel(const __grid_constant__ PParams p) {
+    using C = Cfg<HD, FMT, QL>;
+    constexpr int NQ = C::NQ, NSB = C::NSB, NSLOT = C::NSLOT, KL = C::KL, DV = C::DV, NCONST = C::NCONST;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t *sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t *sm = smem_raw;
     const uint32_t sm_u32 = smem_u32(sm);
-    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(sm + OFF_MISC);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + OFF_MISC + 4);
-    float *xch = reinterpret_cast<float *>(sm + OFF_XCH);              // [3][TPR][128]
-    const uint32_t bar0 = sm_u32 + OFF_BAR;
-    auto bar_raw_full = [&](int s) { return bar0 + 8 * s; };            // TMA -> dequant and MMA (tx bytes)
-    auto bar_raw_empty = [&](int s) { return bar0 + 8 * (2 + s); };     // dequant warps (V converted) + commit after QK (1) + softmax warps (scales used) -> TMA
-    const uint32_t bar_v16_full = bar0 + 8 * 4;                         // dequant warps -> MMA
-    const uint32_t bar_v16_empty = bar0 + 8 * 5;                        // commit after PV -> dequant
-    const uint32_t bar_s_full = bar0 + 8 * 6;                           // commit after QK -> softmax
-    const uint32_t bar_s_empty = bar0 + 8 * 7;                          // softmax warps: S is in registers -> MMA
-    const uint32_t bar_p_full = bar0 + 8 * 8;                           // softmax warps -> MMA
-    const uint32_t bar_o_done = bar0 + 8 * 9;                           // commit after PV -> softmax
-    const uint32_t bar_q_ready = bar0 + 8 * 10;                         // softmax warps -> MMA
-    const uint32_t bar_xch = bar0 + 8 * 11;                             // softmax warps: the threads of every row have written their exchange slots
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(sm + C::OFF_MISC);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + C::OFF_MISC + 4);
+    const uint32_t bar0 = sm_u32 + C::OFF_BAR;
+    auto bar_full = [&](int s) { return bar0 + 8 * s; };                          // dequant warps -> MMA
+    auto bar_empty = [&](int s) { return bar0 + 8 * (NSLOT + s); };               // commit after the slot's last product -> dequant
+    auto bar_const = [&](int i) { return bar0 + 8 * (2 * NSLOT + i); };           // dequant warps -> softmax: a tile's per-key constants
+    auto bar_s_full = [&](int i) { return bar0 + 8 * (2 * NSLOT + NCONST + i); }; // commit after QK -> softmax
+    auto bar_p_full = [&](int i) { return bar0 + 8 * (2 * NSLOT + NCONST + NSB + i); };      // softmax warps -> MMA
+    auto bar_o_done = [&](int i) { return bar0 + 8 * (2 * NSLOT + NCONST + 2 * NSB + i); };  // commit after PV -> softmax (index: S buffer)
+    const uint32_t bar_q_ready = bar0 + 8 * (2 * NSLOT + NCONST + 3 * NSB);       // softmax warps -> MMA
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // heavy blocks (late query positions: the most key tiles) are scheduled first
-    const int qb = p.q_blocks - 1 - blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-    const int s_first = qb * p.pos_per_cta;
-    const int s_last = min(p.S, s_first + p.pos_per_cta) - 1;
+    // one-dimensional grid, heaviest work first: late query blocks (the most key tiles) of every KV head before earlier ones
+    int bid = blockIdx.x;
+    const int dpart = C::DSPLIT > 1 ? bid % C::DSPLIT : 0;
+    bid /= C::DSPLIT;
+    const int kvh = bid % p.nkv;
+    bid /= p.nkv;
+    const int b = bid % p.batch, qb = p.q_blocks - 1 - bid / p.batch;
 
-    // key range of the block: from the first row's lower bound to the last row's upper bound
-    const int hi_blk = min(p.d0 + s_last, p.key_len - 1);
-    const int lo_blk = p.window > 0 ? max(0, p.d0 + s_first - p.window + 1) : 0;
-    const int tile_lo = lo_blk / KT;
-    const int n_tiles = hi_blk >= lo_blk ? hi_blk / KT - tile_lo + 1 : 0;
-    const int map_row0 = kvh * p.cache_cap + p.row0;                   // row of key index 0 in the tensor maps
+    // key range of each query tile (whole key tiles), and of the CTA
+    int g_first[NQ], g_last[NQ];                       // tiles of query tile g, relative to the CTA's first (empty: first > last)
+    int tile_lo = 0x7fffffff, tile_hi = -1;
+#pragma unroll
+    for (int g = 0; g < NQ; ++g) {
+        const int s_first = (qb * NQ + g) * p.pos_per_tile;
+        const int s_last = min(p.S, s_first + p.pos_per_tile) - 1;
+        const int hi = s_last >= s_first ? min(p.d0 + s_last, p.key_len - 1) : -1;
+        const int lo = p.window > 0 ? max(0, p.d0 + s_first - p.window + 1) : 0;
+        if (hi >= lo) {
+            g_first[g] = lo / KT; g_last[g] = hi / KT;
+            tile_lo = min(tile_lo, g_first[g]); tile_hi = max(tile_hi, g_last[g]);
+        } else {
+            g_first[g] = 0x3fffffff; g_last[g] = -1;
+        }
+    }
+    const int n_tiles = tile_hi >= 0 ? tile_hi - tile_lo + 1 : 0;
+    if (n_tiles == 0) tile_lo = 0;
+#pragma unroll
+    for (int g = 0; g < NQ; ++g) { g_first[g] -= tile_lo; g_last[g] -= tile_lo; }
+    // (consecutive query tiles have overlapping or adjacent ranges, so every tile of the CTA serves at least one of them;
+    // a tile that serves none, possible only with a window shorter than a query tile's span, costs its slots and no products)
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        fused::mbar_init(bar_raw_full(0), 1); fused::mbar_init(bar_raw_full(1), 1);
-        fused::mbar_init(bar_raw_empty(0), NSOFT / 32 + 3); fused::mbar_init(bar_raw_empty(1), NSOFT / 32 + 3);
-        fused::mbar_init(bar_v16_full, 2); fused::mbar_init(bar_v16_empty, 1);
-        fused::mbar_init(bar_s_full, 1); fused::mbar_init(bar_s_empty, NSOFT / 32);
-        fused::mbar_init(bar_p_full, NSOFT / 32); fused::mbar_init(bar_o_done, 1);
-        fused::mbar_init(bar_q_ready, NSOFT / 32);
-        fused::mbar_init(bar_xch, NSOFT / 32);
+        for (int s = 0; s < NSLOT; ++s) { fused::mbar_init(bar_full(s), 2); fused::mbar_init(bar_empty(s), 1); }
+        for (int i = 0; i < NCONST; ++i) fused::mbar_init(bar_const(i), 2);
+        for (int i = 0; i < NSB; ++i) { fused::mbar_init(bar_s_full(i), 1); fused::mbar_init(bar_p_full(i), 8); fused::mbar_init(bar_o_done(i), 1); }
+        fused::mbar_init(bar_q_ready, C::NSW);
         fused::fence_mbar_init();
     }
-    // the scale stages start as zeros: a partial copy at the end of the key array then leaves finite values behind
-    for (int e = threadIdx.x; e < 2 * 2 * KT; e += NTHREADS) reinterpret_cast<float *>(sm + OFF_SC)[e] = 0.0f;
-    fused::fence_proxy_async();
-    if (warp == W_MMA && lane == 0) { fused::prefetch_tensormap(&tm.k); fused::prefetch_tensormap(&tm.v); }
-    if (warp == W_TMA) {
-        tc5::tmem_alloc(sm_u32 + OFF_MISC, TMEM_COLS);
+    if (warp == C::W_MMA) {
+        tc5::tmem_alloc(sm_u32 + C::OFF_MISC, 512);
         tc5::tmem_relinquish();
     }
     tc5::tc_fence_before();
@@ -226,331 +304,527 @@ __global__ void __launch_bounds__(NTHREADS, 1) attn_prefill_kernel(const __grid_
     fused::pdl_wait();                         // the query and the cache rows may come from the stream predecessor
     fused::pdl_launch_dependents();
 
-    if (warp == W_TMA) {
-        // =========================================================== TMA producer
-        if (lane == 0) {
-            for (int i = 0; i < n_tiles; ++i) {
-                const int st = i & 1;
-                if (i >= 2 && !wait_or_abort(bar_raw_empty(st), ((i >> 1) - 1) & 1, abort_flag, p.fault)) break;
-                const uint32_t dst = sm_u32 + OFF_RAW + st * 2 * RAW_TILE;
-                const int row = map_row0 + (tile_lo + i) * KT;
-                // the tile's fp32 row scales ride along as two bulk copies (whole 16-byte units inside the key array)
-                const int t0 = (tile_lo + i) * KT;
-                const uint32_t sc_bytes = p.scales_vec ? (uint32_t)(min(KT, p.key_len - t0) & ~3) * 4u : 0u;
-                fused::mbar_expect_tx(bar_raw_full(st), 2 * RAW_TILE + 2 * sc_bytes);
-                fused::tma_load_tile(dst, &tm.k, row, b, bar_raw_full(st));
-                fused::tma_load_tile(dst + RAW_TILE, &tm.v, row, b, bar_raw_full(st));
-                if (sc_bytes) {
-                    const size_t so = b * (p.scale_batch_stride / 4) + (size_t)kvh * p.cache_cap + p.row0 + t0;
-                    fused::bulk_load(sm_u32 + OFF_SC + st * 2 * KT * 4, p.k_scales + so, sc_bytes, bar_raw_full(st));
-                    fused::bulk_load(sm_u32 + OFF_SC + st * 2 * KT * 4 + KT * 4, p.v_scales + so, sc_bytes, bar_raw_full(st));
+    if (warp == C::W_MMA) {
+        // =========================================================== MMA issuer: one elected lane walks the schedule
+        if (elect_one()) {
+        constexpr uint32_t idesc_qk = make_idesc_f16(KT, false), idesc_pv = make_idesc_f16(128, true);
+        const uint64_t qdesc = tc5::smem_desc_sw128(sm_u32 + C::OFF_Q);
+        const uint64_t rdesc = tc5::smem_desc_sw128(sm_u32 + C::OFF_RING);
+        // V operand, MN-major: the two 64-dim blocks of a slot are one operand, the second BLOCK bytes after the first
+        // (leading-dimension offset); key groups of 8 rows stay 1024 bytes apart
+        const uint64_t vrdesc = (rdesc & ~(0x3fffull << 16)) | ((uint64_t)(C::BLOCK >> 4) << 16);
+        // the next unit of the ring: its first slot (a unit's KL slots share one pair of barriers, the first slot's)
+        int ring = 0;
+        uint32_t ring_phase = 0;
+        auto next_unit = [&](int &slot) {
+            slot = ring;
+            const bool ok = wait_or_abort(bar_full(ring), ring_phase, abort_flag, p.fault);
+            tc5::tc_fence_after();
+            ring += KL;
+            if (ring == NSLOT) { ring = 0; ring_phase ^= 1u; }
+            return ok;
+        };
+        auto commit = [&](uint32_t bar) { tc5::umma_commit(bar); };
+        // S buffer buf += dims 128 c .. 128 c + 127 of query tile g x the K slots from n on
+        auto qk = [&](int g, int buf, int c, int n) {
+            const uint32_t d = tmem_base + C::TMEM_S + buf * KT;
+            {
+#pragma unroll
+                for (int kl = 0; kl < KL; ++kl) {
+                    const uint64_t bd = rdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
+#pragma unroll
+                    for (int ql = 0; ql < QL; ++ql) {
+                        if (ql + kl > 1) continue;                     // low x low: 2^-18 of the logit's terms and less
+                        const uint64_t ad = qdesc + (uint64_t)(((g * QL + ql) * C::Q_LIMB + 2 * c * C::Q_BLOCK) >> 4);
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            umma_f16(d, ad + (uint64_t)(((k >> 2) * C::Q_BLOCK >> 4) + (k & 3) * 2), bd + (uint64_t)(((k >> 2) * C::BLOCK >> 4) + (k & 3) * 2),
+                                     idesc_qk, (c | kl | ql | k) != 0 ? 1u : 0u);
+                    }
                 }
             }
-        }
-        __syncwarp();
-    } else if (warp == W_MMA) {
-        // =========================================================== MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_qk = tc5::make_idesc(KT, true, true, false);
-            const uint32_t idesc_pv = make_idesc_f16(HD, true);
-            const uint64_t qdesc[2] = {tc5::smem_desc_sw128(sm_u32 + OFF_Q8), tc5::smem_desc_sw128(sm_u32 + OFF_Q8 + RAW_TILE)};
-            const uint64_t pdesc[2] = {tc5::smem_desc_sw128(sm_u32 + OFF_P16), tc5::smem_desc_sw128(sm_u32 + OFF_P16 + H_TILE)};
-            // B of PV, MN-major: the two 64-dim blocks of V16 are one operand, the second H_BLOCK bytes after the first
-            // (leading-dimension offset); key groups of 8 rows stay 1024 bytes apart
-            const uint64_t vdesc = (tc5::smem_desc_sw128(sm_u32 + OFF_V16) & ~(0x3fffull << 16)) | ((uint64_t)(H_BLOCK >> 4) << 16);
-            bool go = n_tiles > 0 && wait_or_abort(bar_q_ready, 0, abort_flag, p.fault);
-            for (int i = 0; go && i <= n_tiles; ++i) {
-                if (i < n_tiles) {
-                    // S_hi / S_lo = Qlimb x K_i^T straight off the bytes TMA wrote: per limb 4 steps of 32 dims (32 bytes)
-                    const int st = i & 1;
-                    if (!wait_or_abort(bar_raw_full(st), (i >> 1) & 1, abort_flag, p.fault)) break;
-                    if (i >= 1 && !wait_or_abort(bar_s_empty, (i - 1) & 1, abort_flag, p.fault)) break;
-                    tc5::tc_fence_after();
-                    const uint64_t kdesc = tc5::smem_desc_sw128(sm_u32 + OFF_RAW + st * 2 * RAW_TILE);
+        };
+        // dims 128 c .. of O of query tile g += P in S buffer buf x the V slots from n on
+        auto pv = [&](int g, int buf, int c, int n, bool first) {
+            const uint32_t a = tmem_base + C::TMEM_S + buf * KT;
+            {
 #pragma unroll
-                    for (int limb = 0; limb < 2; ++limb)
+                for (int kl = 0; kl < KL; ++kl) {
+                    const uint64_t bd = vrdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
 #pragma unroll
-                        for (int k = 0; k < HD / 32; ++k)
-                            tc5::umma_i8(tmem_base + 128 * limb, qdesc[limb] + 2 * k, kdesc + 2 * k, idesc_qk, k > 0);
-                    tc5::umma_commit(bar_s_full);
-                    tc5::umma_commit(bar_raw_empty(st));
-                }
-                if (i >= 1) {
-                    // O += Phi_j x V_j + Plo_j x V_j: per weight limb 8 steps of 16 keys against all 128 dims (an instruction
-                    // costs the issuing thread about a hundred cycles whatever its size: few and large)
-                    // (A: 32 bytes inside a 64-key block, then the next block; B: 16 rows of the MN-major V blocks = 2048 bytes)
-                    const int j = i - 1;
-                    if (!wait_or_abort(bar_v16_full, j & 1, abort_flag, p.fault)) break;
-                    if (!wait_or_abort(bar_p_full, j & 1, abort_flag, p.fault)) break;
-                    tc5::tc_fence_after();
+                    for (int pl = 0; pl < 2; ++pl) {
+                        if (pl + kl > 1) continue;
 #pragma unroll
-                    for (int limb = 0; limb < 2; ++limb)
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            const uint64_t a_adv = (uint64_t)((k >> 2) * (H_BLOCK >> 4) + (k & 3) * 2);
-                            const uint64_t b_adv = (uint64_t)(k * (2048 >> 4));
-                            umma_f16(tmem_base + 256, pdesc[limb] + a_adv, vdesc + b_adv, idesc_pv, (j > 0 || limb > 0 || k > 0) ? 1u : 0u);
-                        }
-                    tc5::umma_commit(bar_v16_empty);
-                    tc5::umma_commit(bar_o_done);
+                        for (int k = 0; k < KT / 16; ++k)              // 16 keys: 8 columns of A, 2048 bytes of the MN-major blocks
+                            umma_f16_ts(tmem_base + C::TMEM_O + g * DV + c * 128, a + 32 * pl + 8 * k, bd + (uint64_t)(k * (2048 >> 4)),
+                                        idesc_pv, (!first || kl || pl || k) ? 1u : 0u);
+                    }
                 }
             }
+        };
+        auto wait_bar = [&](uint32_t bar, uint32_t parity) {
+            const bool ok = wait_or_abort(bar, parity, abort_flag, p.fault);
+            tc5::tc_fence_after();
+            return ok;
+        };
+        bool go = n_tiles > 0 && wait_bar(bar_q_ready, 0);
+        // Ring order K0 K1 V0 K2 V1 ...: with two S buffers per query tile the products of tile i + 1 are done before the
+        // softmax of tile i is, and QK(i + 2) reuses the buffer of PV(i) right behind it (products of one thread run in order).
+        // Buffer and barrier phase follow the query tile's own count of tiles.
+        auto active = [&](int g, int i) { return i >= g_first[g] && i <= g_last[g]; };
+        auto buffer = [&](int g, int i) { return 2 * g + ((i - g_first[g]) & 1); };
+        auto qk_tile = [&](int j) {
+#pragma unroll 1
+            for (int c = 0; c < HD / 128; ++c) {
+                int n;
+                if (!next_unit(n)) return false;
+#pragma unroll
+                for (int g = 0; g < NQ; ++g)
+                    if (active(g, j)) {
+                        qk(g, buffer(g, j), c, n);
+                        if (c == HD / 128 - 1) commit(bar_s_full(buffer(g, j)));
+                    }
+                commit(bar_empty(n));
+            }
+            return true;
+        };
+        go = go && qk_tile(0);
+        if (go && n_tiles > 1) go = qk_tile(1);
+        for (int i = 0; go && i < n_tiles; ++i) {
+            if constexpr (NQ == 2) {
+                // one V unit and one K unit: QK of a query tile goes out behind its PV, before the other tile's weights are waited for
+                int nv, nk = 0;
+                const bool more = i + 2 < n_tiles;
+                if (!(go = next_unit(nv))) break;
+#pragma unroll
+                for (int g = 0; g < NQ; ++g) {
+                    if (go && active(g, i)) {
+                        go = wait_bar(bar_p_full(buffer(g, i)), ((i - g_first[g]) >> 1) & 1);
+                        if (go) { pv(g, buffer(g, i), 0, nv, i == g_first[g]); commit(bar_o_done(buffer(g, i))); }
+                    }
+                    if (g == 1) commit(bar_empty(nv));
+                    if (go && more) {
+                        if (g == 0) go = next_unit(nk);
+                        if (go && active(g, i + 2)) { qk(g, buffer(g, i + 2), 0, nk); commit(bar_s_full(buffer(g, i + 2))); }
+                    }
+                }
+                if (go && more) commit(bar_empty(nk));
+            } else {
+                if (!(go = wait_bar(bar_p_full(buffer(0, i)), (i >> 1) & 1))) break;
+#pragma unroll 1
+                for (int c = 0; c < DV / 128; ++c) {
+                    int n;
+                    if (!(go = next_unit(n))) break;
+                    pv(0, buffer(0, i), c, n, i == 0);
+                    commit(bar_empty(n));
+                }
+                if (!go) break;
+                commit(bar_o_done(buffer(0, i)));
+                if (i + 2 < n_tiles) go = qk_tile(i + 2);
+            }
+        }
         }
         __syncwarp();
-    } else if (warp >= W_DEQ) {
-        // =========================================================== dequant warps: a thread converts key rows t, t + 64 of the V tile
-        const int t = threadIdx.x - NSOFT;
-        for (int i = 0; i < n_tiles; ++i) {
-            const int st = i & 1;
-            const uint8_t *raw = sm + OFF_RAW + st * 2 * RAW_TILE + RAW_TILE;
-            if (!__all_sync(0xffffffffu, wait_or_abort(bar_raw_full(st), (i >> 1) & 1, abort_flag, p.fault))) break;
-            if (i >= 1 && !__all_sync(0xffffffffu, wait_or_abort(bar_v16_empty, (i - 1) & 1, abort_flag, p.fault))) break;
+    } else if (warp >= C::W_DEQ) {
+        // =========================================================== dequant warps: cache bytes -> fp16 operand slots
+        const int team = (warp - C::W_DEQ) >> 1, t = (threadIdx.x - 32 * C::W_DEQ) & 63;
+        const uint8_t *gk = p.k_cache + b * p.kv_batch_stride, *gv = p.v_cache + b * p.kv_batch_stride;
+        const uint8_t *gks = p.k_scales + b * p.scale_batch_stride, *gvs = p.v_scales + b * p.scale_batch_stride;
+        // cache row of key index key (clamped into the array: masked keys then hold finite codes)
+        auto cache_row = [&](int key) {
+            int slot = p.row0 + max(0, min(key, p.key_len - 1));
+            if (slot >= p.cache_cap) slot -= p.cache_cap;
+            return (size_t)kvh * p.cache_cap + slot;
+        };
+        // piece k of this thread: 16-byte piece `ppc` of row prow + k * RSTEP of the slot.  Int8: the 8 lanes of a store
+        // phase take 4 pieces of one 64-dim block from an even and from an odd row, whose swizzled chunks interleave (no
+        // bank conflict).  RSTEP is a multiple of 8 rows: the swizzle is the same for every k
+        const int prow = FMT == KV_I8 ? (t >> 5) * 4 + ((t >> 2) & 1) + 2 * ((t >> 4) & 1) : t >> 2;
+        const int ppc = FMT == KV_I8 ? (t & 3) + 4 * ((t >> 3) & 1) : t & 3;
+        constexpr int RSTEP = FMT == KV_I8 ? 8 : 16;
+        static_assert(RSTEP % 8 == 0, "swizzle period");
+        // byte offsets of the piece's 8-dim chunks inside a slot
+        constexpr int NCH = C::CPP / 8;
+        int soff[NCH];
 #pragma unroll
-            for (int rr = 0; rr < 2; ++rr) {
-                const int r = t + 64 * rr;
+        for (int e = 0; e < NCH; ++e) soff[e] = op_off(prow, NCH * ppc + e, C::BLOCK);
+        // unit i of the ring order K0 K1 V0 K2 V1 ...: V tile or K tile, and which 128 dims
+        constexpr int KU = HD / 128, VU = DV / 128;
+        struct Unit { int tile, v, c; };
+        auto unit_at = [&](int i) {
+            const int lead = KU * min(n_tiles, 2);
+            if (i < lead) return Unit{i / KU, 0, i % KU};
+            i -= lead;
+            const int body = (KU + VU) * max(0, n_tiles - 2);
+            if (i < body) {
+                const int q = i / (KU + VU), r = i % (KU + VU);
+                return r < VU ? Unit{q, 1, r} : Unit{q + 2, 0, r - VU};
+            }
+            i -= body;
+            return Unit{max(0, n_tiles - 2) + i / VU, 1, i % VU};
+        };
+        constexpr int NBW = C::NBW, NP = C::NP, TEAMS = C::TEAMS;
+        constexpr int NSC = FMT == KV_I4B32 ? NP : 1, NCW = FMT == KV_I4B32 ? NBW : 1;
+        // cache bytes of the team's next unit; with the first K unit of a tile the scales of key t of the tile
+        uint4 x[NP];
+        uint32_t sc[NSC], ckw[NCW], cvw[NCW];
+        auto fetch = [&](Unit u) {
+            const uint8_t *base = u.v ? gv : gk;
+            const int key0 = (tile_lo + u.tile) * KT;
+            const int dim0 = (u.v ? dpart * DV : 0) + u.c * 128;       // first dim of the slot
+            const uint8_t *col = base + (FMT == KV_I8 ? dim0 : dim0 / 2) + 16 * ppc;
+            // block-32: the piece is one block; the word that holds its fp16 scale
+            const uint8_t *scol = (u.v ? gvs : gks) + ((dim0 >> 5) + ppc) / 2 * 4;
+            int slot = p.row0 + key0;
+            if (slot >= p.cache_cap) slot -= p.cache_cap;
+            if (key0 + KT <= p.key_len && slot + KT <= p.cache_cap) {  // a whole tile in consecutive rows
+                const size_t cr = (size_t)kvh * p.cache_cap + slot + prow;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {                          // 16 codes per step -> two 16-byte chunks of fp16
-                    const uint4 x = *reinterpret_cast<const uint4 *>(raw + (r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
+                for (int k = 0; k < NP; ++k) {
+                    x[k] = __ldcg(reinterpret_cast<const uint4 *>(col + cr * p.row_bytes + (size_t)(k * RSTEP) * p.row_bytes));
+                    if constexpr (FMT == KV_I4B32) sc[k] = __ldcg(reinterpret_cast<const uint32_t *>(scol + (cr + k * RSTEP) * (NBW * 4)));
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                    const size_t cr = cache_row(key0 + prow + k * RSTEP);
+                    x[k] = __ldcg(reinterpret_cast<const uint4 *>(col + cr * p.row_bytes));
+                    if constexpr (FMT == KV_I4B32) sc[k] = __ldcg(reinterpret_cast<const uint32_t *>(scol + cr * (NBW * 4)));
+                }
+            }
+            if (!u.v && u.c == 0) {
+                const size_t cr = cache_row(key0 + t);
+#pragma unroll
+                for (int w = 0; w < NCW; ++w) {
+                    ckw[w] = __ldcg(reinterpret_cast<const uint32_t *>(gks) + cr * NCW + w);
+                    cvw[w] = __ldcg(reinterpret_cast<const uint32_t *>(gvs) + cr * NCW + w);
+                }
+            }
+        };
+        auto store_const = [&](int tile) {                 // per-key constants of the tile (block-32: with the shifts the conversion reads back)
+            float *cc = reinterpret_cast<float *>(sm + C::OFF_CONST) + (tile % NCONST) * 3 * KT;
+            if constexpr (FMT == KV_I4B32) {
+                const int sk = b32_shift(ckw), sv = b32_shift(cvw);
+                cc[t] = pow2i(-sk);
+                cc[KT + t] = (float)(-sv);
+                cc[2 * KT + t] = pow2i(sv);
+            } else {
+                const float vs = fmaxf(__uint_as_float(cvw[0]), VS_MIN);
+                cc[t] = __uint_as_float(ckw[0]);
+                cc[KT + t] = lg2f(vs);
+                cc[2 * KT + t] = 1.0f / vs;
+            }
+            __syncwarp();
+            if (lane == 0) tc5::mbar_arrive(bar_const(tile % NCONST));
+        };
+        static_assert(KT == 64, "a team's 64 threads take one key each");
+        auto convert = [&](Unit u, int slot) {
+            uint8_t *s0 = sm + C::OFF_RING + slot * C::SLOT;
+            uint8_t *s1 = s0 + (KL - 1) * C::SLOT;
+            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (u.tile % NCONST) * 3 * KT;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const int row = prow + k * RSTEP, koff = k * RSTEP * 128;
+                const uint32_t w[4] = {x[k].x, x[k].y, x[k].z, x[k].w};
+                if constexpr (FMT == KV_I8) {
                     uint4 y0, y1;
-                    cvt4(x.x, y0.x, y0.y); cvt4(x.y, y0.z, y0.w);
-                    cvt4(x.z, y1.x, y1.y); cvt4(x.w, y1.z, y1.w);
-                    *reinterpret_cast<uint4 *>(sm + OFF_V16 + h_off(r, 2 * c)) = y0;
-                    *reinterpret_cast<uint4 *>(sm + OFF_V16 + h_off(r, 2 * c + 1)) = y1;
+                    cvt4(w[0], y0.x, y0.y); cvt4(w[1], y0.z, y0.w);
+                    cvt4(w[2], y1.x, y1.y); cvt4(w[3], y1.z, y1.w);
+                    *reinterpret_cast<uint4 *>(s0 + soff[0] + koff) = y0;
+                    *reinterpret_cast<uint4 *>(s0 + soff[1] + koff) = y1;
+                } else {
+                    uint32_t hi2 = 0, lo2 = 0;
+                    if constexpr (FMT == KV_I4B32) {
+                        const uint32_t bits = (ppc & 1) ? sc[k] >> 16 : sc[k] & 0xffffu;        // (slots start at even blocks)
+                        // the row's power of two: 1 / logit factor for K, 1 / value scale for V
+                        const float up = u.v ? cc[2 * KT + row] : __uint_as_float(0x7f000000u - __float_as_uint(cc[row]));
+                        const float sf = __half2float(__ushort_as_half((unsigned short)bits)) * up;
+                        const float sh = __uint_as_float(__float_as_uint(sf) & 0xfffe0000u);       // top 7 significant bits
+                        hi2 = pack_f16x2(sh, sh);
+                        lo2 = pack_f16x2(sf - sh, sf - sh);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        uint32_t h[4];
+                        cvt8_i4(w[e], h);
+                        const int off = soff[e] + koff;
+                        if constexpr (FMT == KV_I4B32) {
+                            *reinterpret_cast<uint4 *>(s0 + off) = make_uint4(hmul2_u32(h[0], hi2), hmul2_u32(h[1], hi2), hmul2_u32(h[2], hi2), hmul2_u32(h[3], hi2));
+                            *reinterpret_cast<uint4 *>(s1 + off) = make_uint4(hmul2_u32(h[0], lo2), hmul2_u32(h[1], lo2), hmul2_u32(h[2], lo2), hmul2_u32(h[3], lo2));
+                        } else {
+                            *reinterpret_cast<uint4 *>(s0 + off) = make_uint4(h[0], h[1], h[2], h[3]);
+                        }
+                    }
                 }
             }
+        };
+        const int n_units = n_tiles * ((HD + DV) / 128);
+        auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, p.fault)) != 0; };
+        // this team's units are team, team + TEAMS, ...; its next one is on the way while the other teams' are converted
+        Unit u = unit_at(team);
+        if (team < n_units) fetch(u);
+        for (int i = team; i < n_units; i += TEAMS) {
+            const int n = i * KL, lap = n / NSLOT, slot = n - lap * NSLOT;
+            if (lap > 0 && !wait_all(bar_empty(slot), (lap - 1) & 1)) break;
+            if (!u.v && u.c == 0) store_const(u.tile);     // (behind the wait: see nconst)
+            // (the shifts of the tile come from another thread, most often of another team)
+            if (FMT == KV_I4B32 && !wait_all(bar_const(u.tile % NCONST), (u.tile / NCONST) & 1)) break;
+            convert(u, slot);
             fused::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) { tc5::mbar_arrive(bar_v16_full); tc5::mbar_arrive(bar_raw_empty(st)); }
+            if (lane == 0) tc5::mbar_arrive(bar_full(slot));
+            if (i + TEAMS < n_units) {
+                u = unit_at(i + TEAMS);
+                fetch(u);
+            }
         }
+        __syncwarp();
     } else {
-        // =========================================================== softmax warps: four threads per query row
-        const int qt = warp >> 2;                                      // which 32 keys of a tile (and which 32 dims of Q / O) this thread takes
-        const int r = 32 * (warp & 3) + lane;                          // query row = TMEM lane
-        const int s = s_first + r / p.kvg, j = r - (r / p.kvg) * p.kvg;
-        const bool valid = r < p.pos_per_cta * p.kvg && s < p.S;
-        const int hi_r = valid ? min(p.d0 + s, p.key_len - 1) : -1;                     // inclusive
-        const int lo_r = (valid && p.window > 0) ? max(0, p.d0 + s - p.window + 1) : 0;
-        const uint32_t tmem_lane = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
+        // =========================================================== softmax warps
+        const int g = NQ == 2 ? warp >> 3 : 0;
+        const int half = (warp >> 2) & 1;                              // which 16 of the 32 lanes
+        const uint32_t tmem_lane = tmem_base + ((uint32_t)(32 * (warp & 3) + 16 * half) << 16);
+        const uint32_t tmem_o = tmem_lane + C::TMEM_O + g * DV;
         auto wait_warp = [&](uint32_t bar, uint32_t parity) {
             return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, p.fault)) != 0;
         };
-        // Meeting point of the softmax threads: an mbarrier with the same time limit as every other wait (a
-        // hardware barrier would wait forever for a warp that had given up).  false = abandoned.
-        // One arrival per warp: the warp's stores and fences are ordered before it by the warp barrier.
-        auto warp_arrive = [&](uint32_t bar) {
-            __syncwarp();
-            if (lane == 0) tc5::mbar_arrive(bar);
-        };
-        uint32_t xphase = 0;
-        auto pair_sync = [&]() {
-            warp_arrive(bar_xch);
-            const bool ok = wait_warp(bar_xch, xphase);
-            xphase ^= 1u;
-            return ok;
-        };
-        // ---- the query row -> 16-bit fixed point of its own maximum, two int8 limbs (q ~= sq * (256 hi + lo)),
-        // stored K-major in the 128-byte swizzle pattern; this thread converts dims 32 qt .. 32 qt + 31
-        float qscale_r;                          // base-2 logit per unit of the integer dot product and of the key's scale
-        {
-            const long qoff = b * p.q_batch_stride + ((long)(valid ? s : 0) * p.nh + kvh * p.kvg + (valid ? j : 0)) * HD + KPT * qt;
-            float x[KPT];
-#pragma unroll
-            for (int c = 0; c < KPT / 8; ++c) {
-                if (p.q_type == ET_BF16) {
-                    const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(p.q) + qoff) + c);
-                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) { x[8 * c + 2 * e] = __uint_as_float(w[e] << 16); x[8 * c + 2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
-                } else {
-                    const float4 v0 = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.q) + qoff) + 2 * c);
-                    const float4 v1 = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.q) + qoff) + 2 * c + 1);
-                    x[8 * c] = v0.x; x[8 * c + 1] = v0.y; x[8 * c + 2] = v0.z; x[8 * c + 3] = v0.w;
-                    x[8 * c + 4] = v1.x; x[8 * c + 5] = v1.y; x[8 * c + 6] = v1.z; x[8 * c + 7] = v1.w;
-                }
+        // A warp works on 16 rows, a thread on two of them (8 q + lane / 4) and on every fourth pair of keys: a
+        // key's constants cost a shared-memory read per two rows (a row per thread and three constants per key and row
+        // took 1500 of the 4000 cycles of a 64-key step at head_dim 128 on the shared-memory port alone), and four softmax
+        // warps per scheduler cover each other's waits and latencies (two, with 32 rows each: 3300 cycles per step)
+        float qr[2], m[2];                       // logit factor, whole-number running reference
+        F2 l[2];                                 // this thread's share of the denominator
+        int all_lo = 0, all_hi = 0x7fffffff;     // keys that every row of the warp sees
+        const int row0 = 16 * half + (lane >> 2);                      // of the quadrant's 32
+        auto position = [&](int q) { return (qb * NQ + g) * p.pos_per_tile + (32 * (warp & 3) + row0 + 8 * q) / p.kvg; };
+        auto in_use = [&](int q) { return 32 * (warp & 3) + row0 + 8 * q < p.pos_per_tile * p.kvg && position(q) < p.S; };
+        auto key_range = [&](int q, int &lo, int &hi) {                // inclusive
+            const int sr = position(q);
+            hi = 0x7fffffff; lo = 0;             // (rows not in use: zero queries, never stored, not worth masking for)
+            if (in_use(q)) {
+                hi = min(p.d0 + sr, p.key_len - 1);
+                if (p.window > 0) lo = max(0, p.d0 + sr - p.window + 1);
             }
-            float amax = 0.0f;
+        };
 #pragma unroll
-            for (int d = 0; d < KPT; ++d) amax = fmaxf(amax, fabsf(x[d]));
-            xch[(2 * TPR + qt) * 128 + r] = amax;
-            pair_sync();
+        for (int q = 0; q < 2; ++q) {
+            qr[q] = 0.0f;
+            m[q] = M_INIT;
+            l[q] = F2{0.0f, 0.0f};
+            int lo, hi;
+            key_range(q, lo, hi);
+            all_lo = max(all_lo, lo);
+            all_hi = min(all_hi, hi);
+        }
+        all_lo = __reduce_max_sync(0xffffffffu, all_lo);
+        all_hi = __reduce_min_sync(0xffffffffu, all_hi);
+        // ---- the warp's query rows times the power of two that takes a row's maximum to [2^14, 2^15), as one or two fp16
+        // limbs (which of the two types the rows have decides QL).  The lanes share a row (whole lines per load, four rows in
+        // flight, a short loop): a thread per row, eight dims at a time, took 12 us at head_dim 128 and 29 us at 256 before
+        // the first product
+        {
+            constexpr int DPL = HD / 32, RW = QL == 2 ? DPL : DPL / 2, RB = 4;          // dims and 32-bit words per lane; rows in flight
+            const int base_row = 32 * (warp & 3) + 16 * half;
+            auto load_rows = [&](int r0, uint32_t (&x)[RB][RW]) {
 #pragma unroll
-            for (int o = 1; o < TPR; ++o) amax = fmaxf(amax, xch[(2 * TPR + ((qt + o) & (TPR - 1))) * 128 + r]);
-            const float sq = (valid && amax > 0.0f) ? amax * (1.0f / (float)Q_FIX_MAX) : 1.0f;
-            const float inv = 1.0f / sq;
-            qscale_r = valid ? sq * p.q_scale : 0.0f;
+                for (int jj = 0; jj < RB; ++jj) {
+                    const int row = base_row + r0 + jj, sp = (qb * NQ + g) * p.pos_per_tile + row / p.kvg;
+                    const bool use = row < p.pos_per_tile * p.kvg && sp < p.S;
+                    const long off = b * p.q_batch_stride + ((long)sp * p.nh + kvh * p.kvg + row % p.kvg) * HD + DPL * lane;
 #pragma unroll
-            for (int c = 0; c < KPT / 16; ++c) {                       // 16 dims per 16-byte chunk
-                uint32_t wh[4], wl[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    uint32_t ph = 0, pl = 0;
-#pragma unroll
-                    for (int bb = 0; bb < 4; ++bb) {
-                        int qf = valid ? __float2int_rn(x[16 * c + 4 * e + bb] * inv) : 0;
-                        qf = max(-Q_FIX_MAX, min(Q_FIX_MAX, qf));
-                        const int hi = (qf + 128) >> 8, lo = qf - (hi << 8);
-                        ph |= (uint32_t)(hi & 0xff) << (8 * bb);
-                        pl |= (uint32_t)(lo & 0xff) << (8 * bb);
+                    for (int c = 0; c < RW / 2; ++c) {
+                        const uint2 v = use ? __ldcg(reinterpret_cast<const uint2 *>(p.q + off * (QL == 2 ? 4 : 2)) + c) : make_uint2(0u, 0u);
+                        x[jj][2 * c] = v.x; x[jj][2 * c + 1] = v.y;
                     }
-                    wh[e] = ph; wl[e] = pl;
                 }
-                const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((((KPT / 16) * qt + c) ^ (r & 7)) << 4);
-                *reinterpret_cast<uint4 *>(sm + OFF_Q8 + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4 *>(sm + OFF_Q8 + RAW_TILE + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+            };
+            uint32_t cur[RB][RW], nxt[RB][RW];
+            load_rows(0, cur);
+#pragma unroll 1
+            for (int r0 = 0; r0 < 16; r0 += RB) {
+                if (r0 + RB < 16) load_rows(r0 + RB, nxt);
+#pragma unroll
+                for (int jj = 0; jj < RB; ++jj) {
+                    float x[DPL];
+#pragma unroll
+                    for (int d = 0; d < DPL; ++d)
+                        x[d] = __uint_as_float(QL == 2 ? cur[jj][d % RW] : (d & 1) ? cur[jj][d / 2 % RW] & 0xffff0000u : cur[jj][d / 2 % RW] << 16);
+                    float amax = 0.0f;
+#pragma unroll
+                    for (int d = 0; d < DPL; ++d) amax = fmaxf(amax, fabsf(x[d]));
+                    amax = tc5::redux_max(amax);
+                    const int ex = (int)(__float_as_uint(amax) >> 23);                 // biased exponent (0: a zero or denormal row)
+                    const int sh = ex > 0 ? min(126, 14 + 127 - ex) : 0;
+                    const float up = pow2i(sh);
+                    if ((lane >> 2) == ((r0 + jj) & 7)) { if (r0 < 8) qr[0] = pow2i(-sh) * p.q_scale; else qr[1] = pow2i(-sh) * p.q_scale; }
+                    uint8_t *qt = sm + C::OFF_Q + g * QL * C::Q_LIMB;
+                    const int row = base_row + r0 + jj;
+#pragma unroll
+                    for (int c = 0; c < DPL / 4; ++c) {                // 4 dims = half a 16-byte chunk
+                        const int d0 = DPL * lane + 4 * c;
+                        const float x0 = x[4 * c] * up, x1 = x[4 * c + 1] * up, x2 = x[4 * c + 2] * up, x3 = x[4 * c + 3] * up;
+                        const __half2 h0 = __floats2half2_rn(x0, x1), h1 = __floats2half2_rn(x2, x3);
+                        uint8_t *dst = qt + op_off(row, d0 >> 3, C::Q_BLOCK) + (d0 & 4) * 2;
+                        *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
+                        if constexpr (QL == 2)
+                            *reinterpret_cast<uint2 *>(dst + C::Q_LIMB) = make_uint2(pack_f16x2(x0 - __low2float(h0), x1 - __high2float(h0)),
+                                                                                     pack_f16x2(x2 - __low2float(h1), x3 - __high2float(h1)));
+                    }
+                }
+#pragma unroll
+                for (int jj = 0; jj < RB; ++jj)
+#pragma unroll
+                    for (int c = 0; c < RW; ++c) cur[jj][c] = nxt[jj][c];
             }
             fused::fence_proxy_async();
-            warp_arrive(bar_q_ready);
+            __syncwarp();
+            if (lane == 0) tc5::mbar_arrive(bar_q_ready);
         }
-        // fp32 row scales of the keys, read per tile by every thread (the same 1 KB for the whole CTA: L1 hits)
-        const float *gks = p.k_scales + b * (p.scale_batch_stride / 4) + (size_t)kvh * p.cache_cap + p.row0;
-        const float *gvs = p.v_scales + b * (p.scale_batch_stride / 4) + (size_t)kvh * p.cache_cap + p.row0;
-        float m = M_INIT, l = 0.0f;              // running maximum of the row (its threads agree), this thread's share of the denominator
         bool alive = true;
-        for (int i = 0; alive && i < n_tiles; ++i) {
-            const int t0 = (tile_lo + i) * KT + KPT * qt;              // first key of this thread's share of the tile
-            // rows outside [lo_r, hi_r] see nothing of the key (a select, never a multiply); decided per warp, so that
-            // whole tiles in the middle of every row's range carry no masking instructions at all
-            const bool need_mask = __any_sync(0xffffffffu, t0 < lo_r || t0 + KPT - 1 > hi_r);
-            const int st = i & 1;
-            // scales of this thread's keys: in shared memory when they could ride the bulk copies (the copy covers whole
-            // 16-byte units inside the key array: a ragged tail is read from global memory), else from global memory
-            const bool whole = p.scales_vec && (((tile_lo + i) * KT + (min(KT, p.key_len - (tile_lo + i) * KT) & ~3)) >= t0 + KPT);
-            const float *sks = reinterpret_cast<const float *>(sm + OFF_SC + st * 2 * KT * 4) + KPT * qt - t0;      // used when `whole`
-            const float *svs = reinterpret_cast<const float *>(sm + OFF_SC + st * 2 * KT * 4 + KT * 4) + KPT * qt - t0;
-            const int tl = p.key_len - 1;
-            if (!wait_warp(bar_raw_full(st), (i >> 1) & 1)) { alive = false; break; }   // the scales have landed
-            if (!wait_warp(bar_s_full, i & 1)) { alive = false; break; }
+        const int first = NQ == 2 && g == 1 ? g_first[NQ - 1] : g_first[0], last = NQ == 2 && g == 1 ? g_last[NQ - 1] : g_last[0];
+        for (int i = max(first, 0); alive && i <= last; ++i) {
+            const int it = i - first;                                  // this row's tiles so far
+            const int buf = 2 * g + (it & 1);
+            const uint32_t ts = tmem_lane + C::TMEM_S + buf * KT;
+            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (i % NCONST) * 3 * KT;
+            // (the constants were stored before the K slots of the tile: this wait only orders the reads; it may not come
+            // first, a query tile whose range starts late would meet an older phase of the barrier)
+            if (!wait_warp(bar_s_full(buf), (it >> 1) & 1)) { alive = false; break; }
+            if (!wait_warp(bar_const(i % NCONST), (i / NCONST) & 1)) { alive = false; break; }
             tc5::tc_fence_after();
-            float sv[KPT];                                             // base-2 logits of this row against its 32 keys
-            float tmax = -CUDART_INF_F;
-#pragma unroll
-            for (int c = 0; c < KPT / 16; ++c) {                       // 16 columns of each limb at a time: registers
-                int sh[16], sl[16];
-                tmem_ld16i(tmem_lane + KPT * qt + 16 * c, sh);
-                tmem_ld16i(tmem_lane + 128 + KPT * qt + 16 * c, sl);
+            const int t0 = (tile_lo + i) * KT;
+            F2 u[2][KT / 8];                     // [row][pair e: keys 8 e + 2 (lane % 4) + {0, 1}]
+            {
+                uint32_t x[32];
+                tmem_ld_frag64(ts, x);
                 tc5::tmem_wait_ld();
 #pragma unroll
-                for (int e4 = 0; e4 < 16; e4 += 4) {
-                    float4 k4;
-                    if (whole) {
-                        k4 = *reinterpret_cast<const float4 *>(sks + t0 + 16 * c + e4);
-                    } else {
-                        k4 = make_float4(gks[min(t0 + 16 * c + e4, tl)], gks[min(t0 + 16 * c + e4 + 1, tl)], gks[min(t0 + 16 * c + e4 + 2, tl)],
-                                         gks[min(t0 + 16 * c + e4 + 3, tl)]);
+                for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(x[e]));          // no use above the wait
+#pragma unroll
+                for (int e = 0; e < KT / 8; ++e)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) u[q][e] = F2{__uint_as_float(x[4 * e + 2 * q]), __uint_as_float(x[4 * e + 2 * q + 1])};
+            }
+            const F2 *cc2 = reinterpret_cast<const F2 *>(cc) + (lane & 3);
+            float cm[2] = {-CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+            for (int e = 0; e < KT / 8; ++e) {
+                const F2 a = cc2[4 * e], d = cc2[KT / 2 + 4 * e];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) u[q][e] = fma2(mul2(u[q][e], a), F2{qr[q], qr[q]}, d);
+            }
+            // rows outside their range see nothing of a key (a select, never a multiply); tiles inside every row's range
+            // carry no masking instructions at all
+            if (t0 < all_lo || t0 + KT - 1 > all_hi) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    int lo, hi;
+                    key_range(q, lo, hi);
+#pragma unroll
+                    for (int e = 0; e < KT / 8; ++e) {
+                        const int t = t0 + 8 * e + 2 * (lane & 3);
+                        u[q][e].x = (t >= lo && t <= hi) ? u[q][e].x : -CUDART_INF_F;
+                        u[q][e].y = (t + 1 >= lo && t + 1 <= hi) ? u[q][e].y : -CUDART_INF_F;
                     }
-                    const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
+                }
+            }
+            bool moved = false;
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // limb sums are below 128 * 128 * 127 < 2^22: 256 hi + lo fits an int, one rounding in the conversion
-                        float u = (float)(sh[e4 + e] * 256 + sl[e4 + e]) * (qscale_r * kk[e]);
-                        if (need_mask) {
-                            const int t = t0 + 16 * c + e4 + e;
-                            u = (t >= lo_r && t <= hi_r) ? u : -CUDART_INF_F;
-                        }
-                        sv[16 * c + e4 + e] = u;
-                        tmax = fmaxf(tmax, u);
+            for (int q = 0; q < 2; ++q) {
+#pragma unroll
+                for (int e = 0; e < KT / 8; ++e) cm[q] = fmaxf(cm[q], fmaxf(u[q][e].x, u[q][e].y));
+                moved = moved || cm[q] > m[q] + LAZY;
+            }
+            if (__any_sync(0xffffffffu, moved)) {
+                // the reference of some rows moves, by a whole power of two: denominator and output sums follow
+                float alpha[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    cm[q] = fmaxf(cm[q], __shfl_xor_sync(0xffffffffu, cm[q], 1));
+                    cm[q] = fmaxf(cm[q], __shfl_xor_sync(0xffffffffu, cm[q], 2));
+                    const float m_new = cm[q] > m[q] + LAZY ? ceilf(cm[q]) : m[q];
+                    alpha[q] = m_new == m[q] ? 1.0f : (m[q] - m_new < -126.0f ? 0.0f : pow2i((int)(m[q] - m_new)));
+                    m[q] = m_new;
+                    l[q].x *= alpha[q]; l[q].y *= alpha[q];
+                }
+                if (it > 0) {
+                    if (!wait_warp(bar_o_done(2 * g + ((it - 1) & 1)), ((it - 1) >> 1) & 1)) { alive = false; break; }
+                    tc5::tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < DV / 32; ++c) {
+                        uint32_t x[16];
+                        tmem_ld_frag32(tmem_o + 32 * c, x);
+                        tc5::tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) x[e] = __float_as_uint(__uint_as_float(x[e]) * alpha[(e >> 1) & 1]);
+                        tmem_st_frag32(tmem_o + 32 * c, x);
                     }
                 }
             }
-            tc5::tc_fence_before();
-            warp_arrive(bar_s_empty);                                  // S is in registers: QK of the next tile may overwrite it
-            // the row's tile maximum: its threads meet through shared memory (double-buffered by tile parity)
-            xch[((i & 1) * TPR + qt) * 128 + r] = tmax;
-            if (!pair_sync()) { alive = false; break; }
+            // weights, in place of S: hi limbs in the buffer's first 32 columns, lo limbs in the others (a warp's rows are
+            // its own, and all of their S is in registers)
+            const F2 minus1{-1.0f, -1.0f};
+            uint32_t ph[16], pl[16];
 #pragma unroll
-            for (int o = 1; o < TPR; ++o) tmax = fmaxf(tmax, xch[((i & 1) * TPR + ((qt + o) & (TPR - 1))) * 128 + r]);
-            // the running maximum only moves when the tile exceeds it by more than 2^8: the weights stay below 2^8 and
-            // the accumulator in tensor memory is rescaled a handful of times per row instead of once per tile
-            const bool moved = tmax > m + LAZY;
-            const float m_new = moved ? tmax : m;
-            const float alpha = moved ? ex2f(m - m_new) : 1.0f;
-            m = m_new;
-            // P is single-buffered and O lives in tensor memory: both wait for the previous tile's PV product
-            if (i >= 1 && !wait_warp(bar_o_done, (i - 1) & 1)) { alive = false; break; }
-            if (i >= 1 && __any_sync(0xffffffffu, moved)) {            // this thread rescales its 32 dims of O
-                tc5::tc_fence_after();
-                float o[32];
-                tmem_ld32(tmem_lane + 256 + KPT * qt, o);
+            for (int e = 0; e < KT / 8; ++e) {
+                const F2 iv = cc2[KT + 4 * e];
 #pragma unroll
-                for (int e = 0; e < 32; ++e) o[e] *= alpha;
-                tmem_st32(tmem_lane + 256 + KPT * qt, o);
-                tmem_wait_st();
-            }
-            // weights of this thread's 32 keys = chunks 4 qt .. 4 qt + 3 of the P tiles: weight x value scale as fp16 hi + lo
-            float lsum0 = 0.0f, lsum1 = 0.0f;
-#pragma unroll
-            for (int e8 = 0; e8 < KPT; e8 += 8) {
-                float vv[8];
-                if (whole) {
-                    const float4 a4 = *reinterpret_cast<const float4 *>(svs + t0 + e8);
-                    const float4 b4 = *reinterpret_cast<const float4 *>(svs + t0 + e8 + 4);
-                    vv[0] = a4.x; vv[1] = a4.y; vv[2] = a4.z; vv[3] = a4.w; vv[4] = b4.x; vv[5] = b4.y; vv[6] = b4.z; vv[7] = b4.w;
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) vv[e] = gvs[min(t0 + e8 + e, tl)];
+                for (int q = 0; q < 2; ++q) {
+                    F2 w = add2(u[q][e], F2{-m[q], -m[q]});
+                    w = F2{ex2f(w.x), ex2f(w.y)};
+                    l[q] = fma2(w, iv, l[q]);
+                    const __half2 hh = __floats2half2_rn(w.x, w.y);
+                    ph[2 * e + q] = *reinterpret_cast<const uint32_t *>(&hh);
+                    w = fma2(F2{__low2float(hh), __high2float(hh)}, minus1, w);
+                    pl[2 * e + q] = pack_f16x2(w.x, w.y);
                 }
-                uint32_t wh[4], wl[4];
-#pragma unroll
-                for (int e = 0; e < 8; e += 2) {
-                    const float p0 = ex2f(sv[e8 + e] - m), p1 = ex2f(sv[e8 + e + 1] - m);
-                    lsum0 += p0; lsum1 += p1;
-                    const float w0 = p0 * vv[e], w1 = p1 * vv[e + 1];
-                    const __half2 h = __floats2half2_rn(w0, w1);
-                    const __half2 hl = __floats2half2_rn(w0 - __low2float(h), w1 - __high2float(h));
-                    wh[e >> 1] = *reinterpret_cast<const uint32_t *>(&h);
-                    wl[e >> 1] = *reinterpret_cast<const uint32_t *>(&hl);
-                }
-                const int chunk = (KPT / 8) * qt + (e8 >> 3);          // 16-byte chunk (8 keys) of the row
-                *reinterpret_cast<uint4 *>(sm + OFF_P16 + h_off(r, chunk)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4 *>(sm + OFF_P16 + H_TILE + h_off(r, chunk)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
             }
-            l = fmaf(l, alpha, lsum0 + lsum1);
-            fused::fence_proxy_async();
+            tmem_st_pairs32(ts, ph);
+            tmem_st_pairs32(ts + 32, pl);
+            tmem_wait_st();
             tc5::tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                tc5::mbar_arrive(bar_raw_empty(st));                   // done with the stage's scales
-                tc5::mbar_arrive(bar_p_full);
-            }
+            if (lane == 0) tc5::mbar_arrive(bar_p_full(buf));
         }
-        // ---- output: O / l (rows without any key are exact zeros, lib/batched_attn_gpu.mojo:329-409); this thread
-        // writes dims 32 qt .. 32 qt + 31 of its row
-        if (alive && n_tiles > 0) alive = wait_warp(bar_o_done, (n_tiles - 1) & 1);
-        if (alive) {
-            xch[(2 * TPR + qt) * 128 + r] = l;
-            alive = pair_sync();
-#pragma unroll
-            for (int o = 1; o < TPR; ++o) l += xch[(2 * TPR + ((qt + o) & (TPR - 1))) * 128 + r];
-        }
+        // ---- output: O / l (rows without any key are exact zeros, lib/batched_attn_gpu.mojo:329-409)
+        const int mine = last >= max(first, 0) ? last - first + 1 : 0;
+        // (the barrier's phase before that is known to be over: S of the last tile was issued behind that PV)
+        if (alive && mine > 0) alive = wait_warp(bar_o_done(2 * g + ((mine - 1) & 1)), ((mine - 1) >> 1) & 1);
         if (alive) {
             tc5::tc_fence_after();
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            const long oi = b * p.out_batch_stride + ((long)(valid ? s : 0) * p.nh + kvh * p.kvg + (valid ? j : 0)) * HD + KPT * qt;
-            float o[32];
-            if (n_tiles > 0) {
-                tmem_ld32(tmem_lane + 256 + KPT * qt, o);
-            } else {
+            float inv[2];
+            long oi[2];
+            bool vr[2];
 #pragma unroll
-                for (int e = 0; e < 32; ++e) o[e] = 0.0f;
+            for (int q = 0; q < 2; ++q) {
+                float x = l[q].x + l[q].y;
+                x += __shfl_xor_sync(0xffffffffu, x, 1);
+                x += __shfl_xor_sync(0xffffffffu, x, 2);
+                inv[q] = x > 0.0f ? 1.0f / x : (x == x ? 0.0f : x);
+                const int row = 32 * (warp & 3) + row0 + 8 * q;
+                vr[q] = in_use(q);
+                oi[q] = b * p.out_batch_stride + ((long)position(q) * p.nh + kvh * p.kvg + row % p.kvg) * HD + dpart * DV + 2 * (lane & 3);
             }
-            if (valid) {
-                if (p.out_type == ET_BF16) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(p.out) + oi);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const __nv_bfloat162 h = __floats2bfloat162_rn(o[8 * q4 + 2 * e] * inv, o[8 * q4 + 2 * e + 1] * inv);
-                            w[e] = *reinterpret_cast<const uint32_t *>(&h);
-                        }
-                        dst[q4] = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
+#pragma unroll 1
+            for (int c = 0; c < DV / 32; ++c) {
+                uint32_t o[16];
+                if (mine > 0) {
+                    tmem_ld_frag32(tmem_o + 32 * c, o);
+                    tc5::tmem_wait_ld();
                 } else {
-                    float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.out) + oi);
 #pragma unroll
-                    for (int q4 = 0; q4 < 8; ++q4)
-                        dst[q4] = make_float4(o[4 * q4] * inv, o[4 * q4 + 1] * inv, o[4 * q4 + 2] * inv, o[4 * q4 + 3] * inv);
+                    for (int e = 0; e < 16; ++e) o[e] = 0u;
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (!vr[q]) continue;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float x = __uint_as_float(o[4 * e + 2 * q]) * inv[q], y = __uint_as_float(o[4 * e + 2 * q + 1]) * inv[q];
+                        const long at = oi[q] + 32 * c + 8 * e;
+                        if (p.out_type == ET_BF16) *reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(p.out) + at) = __floats2bfloat162_rn(x, y);
+                        else *reinterpret_cast<float2 *>(reinterpret_cast<float *>(p.out) + at) = make_float2(x, y);
+                    }
                 }
             }
         }
@@ -559,7 +833,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attn_prefill_kernel(const __grid_
     // ------------------------------------------------------------ tear-down
     tc5::tc_fence_before();
     __syncthreads();
-    if (warp == W_TMA) tc5::tmem_dealloc(tmem_base, TMEM_COLS);
+    if (warp == C::W_MMA) tc5::tmem_dealloc(tmem_base, 512);
 }
 
 }  // namespace pf

@@ -1,0 +1,115 @@
+"""The query-major prefill kernel over every cache format and head dim it serves, at the edges of its tiles: query tiles
+of 128 rows (two per CTA at head_dim 128), key tiles of 64 or 128 keys, ragged ends, windows, wrapped rings, one and two
+query limbs.  Checked against the oracle's fp64 attention over the same cache bytes.
+
+Tolerance: 2e-4 x RMS per row for fp32 outputs.  The operands carry the codes, the block scales and bf16 queries exactly,
+fp32 queries and weights to 2^-22 of the row's largest, so what is left is ex2.approx (2^-22), the rounding of logits of
+about 100 to 2^-17 and of fp32 sums: a few 1e-5; bf16 outputs add their own rounding (2^-9 of the value, +1 ulp)."""
+import numpy as np
+import pytest
+import torch
+
+from nomos_nvfp4_b200 import ops
+from tests._cases import KVCache, bf16_normal
+from tests._gpu import within
+from tests.test_gpu_attn import build_cache
+from tests.test_gpu_prefill import SENTINEL, run_fused
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-4
+
+
+def served(hd, q_type):
+    return not (hd == 512 and q_type == ops.F32)
+
+
+def check(oracle, c, q, got, *, S, klen, start, window, scale, bf16_out):
+    nh = q.shape[-2]
+    want = oracle.attn_exact(q, c.k, c.v, c.ks, c.vs, c.kv_fmt, nh, c.nkv, c.l_hd, c.cache_hd, c.cache_cap, S=S, window=window,
+                             query_base_pos=start + klen - S, win_lo=start, softmax_scale=scale)
+    assert not np.any(got == SENTINEL)
+    for r in range(S):
+        if bf16_out:
+            tol = np.abs(want[r]) * 2.0 ** -8 + TOL * np.sqrt(np.mean(want[r] ** 2))
+            assert np.all(np.abs(got[r] - want[r]) <= tol), f"row {r}"
+        else:
+            ok, rel = within(got[r], want[r], TOL)
+            assert ok, f"row {r}: {rel:.2e} x RMS"
+
+
+@pytest.mark.parametrize("q_type", [ops.F32, ops.BF16])
+@pytest.mark.parametrize("hd", [128, 256, 512])
+@pytest.mark.parametrize("fmt", ["i8", "i4", "i4b32"])
+@pytest.mark.parametrize("S,klen,window,kvg", [(13, 13, 0, 2), (129, 129, 0, 1), (64, 321, 0, 4), (131, 259, 70, 2), (40, 513, 33, 8)])
+def test_formats_and_head_dims(oracle, fmt, hd, q_type, S, klen, window, kvg):
+    if not served(hd, q_type):
+        pytest.skip("fp32 queries of 512-wide heads run as row groups")
+    rng = np.random.default_rng(S + klen + hd + kvg)
+    nkv = 2
+    c = build_cache(fmt, rng, klen, nkv, hd, cap=klen + 3)
+    q = bf16_normal(rng, (S, nkv * kvg, hd))
+    scale = 1.0 / np.sqrt(hd)
+    got, choice = run_fused(c, q, S=S, klen=klen, window=window, scale=scale, q_type=q_type, out_type=q_type, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    check(oracle, c, q, got[0], S=S, klen=klen, start=0, window=window, scale=scale, bf16_out=q_type == ops.BF16)
+
+
+@pytest.mark.parametrize("hd,fmt,q_type", [(128, "i8", ops.F32), (128, "i4b32", ops.BF16), (256, "i4b32", ops.F32), (512, "i4", ops.BF16)])
+def test_wrapped_ring(oracle, hd, fmt, q_type):
+    """The window's keys run past the end of the ring: rows are addressed one by one."""
+    rng = np.random.default_rng(hd)
+    nkv, kvg, S, klen, start, cap, window = 2, 2, 90, 300, 1111, 333, 211
+    c = build_cache(fmt, rng, klen, nkv, hd, cap=cap, start=start)
+    q = bf16_normal(rng, (S, nkv * kvg, hd))
+    scale = 1.0 / np.sqrt(hd)
+    got, choice = run_fused(c, q, S=S, klen=klen, win_start=start, window=window, scale=scale, q_type=q_type, out_type=q_type, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    check(oracle, c, q, got[0], S=S, klen=klen, start=start, window=window, scale=scale, bf16_out=q_type == ops.BF16)
+
+
+@pytest.mark.parametrize("hd,fmt", [(128, "i8"), (256, "i4"), (512, "i4b32")])
+def test_scales_far_apart(oracle, hd, fmt):
+    """Rows, value rows and query rows whose magnitudes differ by up to 1e6 either way, and logits of thousands: the
+    running reference moves often, and no limb may overflow or flush what matters."""
+    rng = np.random.default_rng(900 + hd)
+    nkv, kvg, S, T = 2, 2, 100, 400
+    c = KVCache(fmt, nkv, T, hd)
+    k, v = bf16_normal(rng, (T, nkv, hd)), bf16_normal(rng, (T, nkv, hd))
+    lim = 3.0 if fmt == "i4b32" else 6.0             # block scales are fp16
+    k *= np.float32(10.0) ** rng.uniform(-1, 1, (T, nkv, 1)).astype(np.float32)
+    v *= np.float32(10.0) ** rng.uniform(-lim, lim, (T, nkv, 1)).astype(np.float32)
+    c.append(k, v, 0)
+    q = bf16_normal(rng, (S, nkv * kvg, hd)) * np.exp2(np.round(rng.uniform(-20, 6, (S, nkv * kvg, 1)))).astype(np.float32)
+    got, choice = run_fused(c, q, S=S, klen=T, scale=1.0 / np.sqrt(hd), q_type=ops.BF16, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    # logits reach several thousand here: their fp32 rounding (2^-12) moves the weights
+    want = oracle.attn_exact(q, c.k, c.v, c.ks, c.vs, c.kv_fmt, nkv * kvg, nkv, hd, hd, T, S=S, query_base_pos=T - S, softmax_scale=1.0 / np.sqrt(hd))
+    for r in range(S):
+        ok, rel = within(got[0][r], want[r], 2e-3)
+        assert ok, f"row {r}: {rel:.2e} x RMS"
+    assert ops.device_faults() == 0
+
+
+def test_a_row_of_infinities_stays_alone(oracle):
+    """One query row is infinite, one NaN: the other rows of the same tile are what they are without them."""
+    rng = np.random.default_rng(31)
+    nkv, kvg, hd, S, T = 2, 2, 128, 64, 200
+    c = build_cache("i8", rng, T, nkv, hd)
+    q = bf16_normal(rng, (S, nkv * kvg, hd))
+    clean, _ = run_fused(c, q, S=S, klen=T, scale=0.09)
+    q[5, 1], q[9, 2, 3] = np.inf, np.nan
+    got, _ = run_fused(c, q, S=S, klen=T, scale=0.09)
+    keep = np.ones((S, nkv * kvg), bool)
+    keep[5, 1] = keep[9, 2] = False
+    assert np.array_equal(got[0][keep], clean[0][keep])
+
+
+@pytest.mark.parametrize("hd,nh,nkv,fmt,S,klen,window,choice", [
+    (256, 32, 16, "i8", 13, 2048, 0, 0), (256, 32, 16, "i8", 1024, 2048, 1024, 2), (256, 32, 16, "i4b32", 24, 16384, 0, 0),
+    (512, 32, 4, "i4b32", 509, 4093, 0, 2), (512, 32, 4, "i8", 16, 16384, 0, 0), (128, 32, 16, "i4", 2048, 2048, 0, 2),
+    (128, 8, 4, "i4b32", 40, 2048, 0, 0), (128, 8, 4, "i8", 40, 2048, 0, 2)])
+def test_which_kernel_takes_a_prompt_chunk(hd, nh, nkv, fmt, S, klen, window, choice):
+    """Few query rows against a long cache run as row groups with split keys, many on the query-major kernel."""
+    a = ops.make_args(q=4096, k_cache=4096, v_cache=4096, k_scales=4096, v_scales=4096, out=4096, kv_fmt={"i8": ops.KV_I8, "i4": ops.KV_I4, "i4b32": ops.KV_I4B32}[fmt],
+                      q_type=ops.BF16, out_type=ops.BF16, S=S, nh=nh, nkv=nkv, kvg=nh // nkv, l_hd=hd, cache_hd=hd, cache_cap=klen, klen=klen, window=window)
+    assert ops.attn_kernel_choice(a) == choice
