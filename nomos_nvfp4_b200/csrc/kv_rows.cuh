@@ -96,4 +96,78 @@ __device__ __forceinline__ float quant_row_i4_block32(const float *src, int l_hd
     return (row_recon > 0.0f) ? __fdiv_rn(row_recon, 127.0f) : 1.0f;
 }
 
+// Largest |x| of the warp in one instruction: the bit patterns of non-negative floats order like the floats, and NaNs count as
+// nothing, as in fmaxf.
+__device__ __forceinline__ float warp_absmax(float x) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fabsf(x), 0.0f))));
+}
+
+// The row codecs above on a row held in registers (lane l has elements l, l + 32, ...): the same roundings, so the
+// same bytes and scales.
+template <int NE>
+__device__ __forceinline__ void quant_regs_i8(const float (&x)[NE], int row_w, int8_t *dst, float *scale_out, int lane) {
+    float a = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) a = fmaxf(a, fabsf(x[k]));
+    a = warp_absmax(a);
+    float scale = __fdiv_rn(a, 127.0f);
+    if (scale == 0.0f) scale = 1.0f;
+    if (lane == 0) *scale_out = scale;
+    const float inv = __fdiv_rn(1.0f, scale);
+#pragma unroll
+    for (int k = 0; k < NE; ++k) dst[lane + 32 * k] = static_cast<int8_t>(round_away_clamp(__fmul_rn(x[k], inv), 127));
+    for (int j = 32 * NE + lane; j < row_w; j += 32) dst[j] = 0;
+}
+// Nibbles of 32 consecutive elements (one per lane) -> 16 bytes; every lane of a group of 8 gets the group's 4 bytes.
+__device__ __forceinline__ uint32_t pack_nibbles(int q, int lane) {
+    uint32_t w = (uint32_t)(q & 0xF) << (4 * (lane & 7));
+    w |= __shfl_xor_sync(0xffffffffu, w, 1);
+    w |= __shfl_xor_sync(0xffffffffu, w, 2);
+    w |= __shfl_xor_sync(0xffffffffu, w, 4);
+    return w;
+}
+template <int NE>
+__device__ __forceinline__ float quant_regs_i4(const float (&x)[NE], int row_w, uint8_t *dst, int lane) {
+    float a = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) a = fmaxf(a, fabsf(x[k]));
+    a = warp_absmax(a);
+    float scale = __fdiv_rn(a, 7.0f);
+    if (scale == 0.0f) scale = 1.0f;
+    const float inv = __fdiv_rn(1.0f, scale);
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+        const uint32_t w = pack_nibbles(round_away_clamp(__fmul_rn(x[k], inv), 7), lane);
+        if ((lane & 7) == 0) *reinterpret_cast<uint32_t *>(dst + 16 * k + (lane >> 1)) = w;
+    }
+    for (int j = 16 * NE + lane; j < row_w / 2; j += 32) dst[j] = 0;
+    return scale;
+}
+template <int NE>
+__device__ __forceinline__ float quant_regs_i4_block32(const float (&x)[NE], uint8_t *dst, __half *scales16, int lane) {
+    float row_recon = 0.0f;
+    // lane b works out block b's scale: one division for the row instead of one per block
+    float amax = 0.0f;
+#pragma unroll
+    for (int b = 0; b < NE; ++b) {
+        const float a = warp_absmax(x[b]);
+        if (lane == b) amax = a;
+    }
+    const float s = (amax > 0.0f) ? __fdiv_rn(amax, 7.0f) : 1.0f;
+    const __half s16 = __float2half_rn(s);
+    const float my_sf = __half2float(s16);
+    if (lane < NE) {
+        scales16[lane] = s16;
+        row_recon = __fmul_rn(my_sf, 7.0f);
+    }
+    row_recon = warp_max(row_recon);
+#pragma unroll
+    for (int b = 0; b < NE; ++b) {
+        const float sf = __shfl_sync(0xffffffffu, my_sf, b);
+        const uint32_t w = pack_nibbles(round_away_clamp(__fdiv_rn(x[b], sf), 7), lane);
+        if ((lane & 7) == 0) *reinterpret_cast<uint32_t *>(dst + 16 * b + (lane >> 1)) = w;
+    }
+    return (row_recon > 0.0f) ? __fdiv_rn(row_recon, 127.0f) : 1.0f;
+}
+
 }  // namespace nomos
