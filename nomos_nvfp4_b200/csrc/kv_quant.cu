@@ -12,6 +12,8 @@
 //   lib/kv_cache_quant.mojo:311-689  int4 appends (row scale, block-32, q8 views)
 //   lib/kv_cache_quant.mojo:708-989  int4 window readers
 //   lib/attention_gpu.mojo:87-162, lib/batched_attn_gpu.mojo:55-102  fp32/bf16 appends
+#include <algorithm>
+
 #include "common.cuh"
 #include "kv_rows.cuh"
 #include "launch.h"
@@ -49,19 +51,31 @@ append_i8_kernel(const float *src_k, const float *src_v, int8_t *dst_k, int8_t *
 
 // Paged int8 caches: one new row per sequence, at position positions[b] of sequence b, i.e. row
 // positions[b] % 128 of page block_table[b][positions[b] / 128]; a page holds 128 rows of every KV head.
+template <bool ROWS128>
 __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32)
 append_paged_i8_kernel(const float *src_k, const float *src_v, int8_t *k_pool, int8_t *v_pool, float *ks_pool, float *vs_pool,
                        const int *block_table, const int *positions, int batch, int nkv, int l_hd, int l_kvd, int max_pages) {
-    const int w = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
-    if (w >= batch * nkv) return;
+    // (between two attention grids, as append_rows_kernel below)
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int row_id = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);             // K rows, then V rows
+    if (row_id >= 2 * batch * nkv) return;
     const int lane = threadIdx.x & 31;
+    const int kv = row_id >= batch * nkv, w = row_id - kv * batch * nkv;
     const int h = w % nkv, b = w / nkv;
+    const float *src = (kv ? src_v : src_k) + (size_t)b * l_kvd + (size_t)h * l_hd;
+    float x[4];
+    if constexpr (ROWS128) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = src[lane + 32 * k];         // on its way while the page is looked up
+    }
     const int pos = positions[b];
     const int page = block_table[(size_t)b * max_pages + pos / 128];
     const size_t row = ((size_t)page * nkv + h) * 128 + (size_t)(pos % 128);
-    const size_t src = (size_t)b * l_kvd + (size_t)h * l_hd;
-    quant_row_i8(src_k + src, l_hd, l_hd, k_pool + row * l_hd, ks_pool + row, lane);
-    quant_row_i8(src_v + src, l_hd, l_hd, v_pool + row * l_hd, vs_pool + row, lane);
+    int8_t *dst = (kv ? v_pool : k_pool) + row * l_hd;
+    float *scale = (kv ? vs_pool : ks_pool) + row;
+    if constexpr (ROWS128) quant_regs_i8<4>(x, 128, dst, scale, lane);
+    else quant_row_i8(src, l_hd, l_hd, dst, scale, lane);
 }
 
 // ------------------------------------------------------------- int4 row codecs
@@ -117,6 +131,39 @@ __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32) append_i4_kernel(AppendI4
     }
 }
 
+// ------------------------------------------------------------- appends of model-sized rows
+// Head dims 128 / 256 / 512 without an int8 view: a warp per (token, KV head, K or V) row, held in registers and read once.
+// Launched with programmatic stream serialization on both sides: a decode step's append is a few KB between two attention
+// grids, whose set-up and settled tiles then overlap it (rows written here are newer than any the next grid may read early).
+// Append + attention, 32q/4kv x 512 block-32 at 32768 keys: 57.4 us with a plain launch, 43.3 so; 9 rows + verify 29.8 / 27.9.
+template <int HD, int FMT>
+__global__ void __launch_bounds__(ROWS_PER_BLOCK * 32) append_rows_kernel(AppendI4Args a) {
+    constexpr int NE = HD / 32;
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const long w = (long)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
+    if (w >= 2l * a.n_s * a.nkv) return;
+    const int lane = threadIdx.x & 31;
+    const int kv = (int)(w & 1), t = (int)(w >> 1);
+    const int h = t % a.nkv, s = t / a.nkv;
+    const float *src = (kv ? a.src_v : a.src_k) + (size_t)s * a.l_kvd + (size_t)h * HD;
+    float x[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) x[k] = src[lane + 32 * k];
+    const size_t row = (size_t)h * a.cache_cap + (size_t)((a.base_pos + s) % a.cache_cap);
+    uint8_t *dst = kv ? a.dst_v : a.dst_k;
+    void *scales = kv ? a.v_scales : a.k_scales;
+    if constexpr (FMT == KV_I8) {
+        quant_regs_i8<NE>(x, a.cache_hd, reinterpret_cast<int8_t *>(dst) + row * a.cache_hd, static_cast<float *>(scales) + row, lane);
+    } else if constexpr (FMT == KV_I4) {
+        const float sc = quant_regs_i4<NE>(x, a.cache_hd, dst + row * (a.cache_hd / 2), lane);
+        if (lane == 0) static_cast<float *>(scales)[row] = sc;
+    } else {
+        const float q8s = quant_regs_i4_block32<NE>(x, dst + row * (a.cache_hd / 2), static_cast<__half *>(scales) + row * NE, lane);
+        if (lane == 0) reinterpret_cast<float *>(static_cast<char *>(scales) + (size_t)a.nkv * a.cache_cap * NE * 2)[row] = q8s;
+    }
+}
+
 // ------------------------------------------------------------- window readers
 // Linear window index j of head h reads ring row h*cache_cap + (win_start+j) % cache_cap
 // and writes linear row h*pitch + j.  One thread converts 8 consecutive elements.
@@ -124,15 +171,14 @@ __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32) append_i4_kernel(AppendI4
 enum ReaderMode { RD_I8_BF16 = 0, RD_I4_BF16 = 1, RD_I4B32_BF16 = 2, RD_I4_Q8 = 3, RD_I4B32_Q8 = 4 };
 
 template <int MODE>
-__global__ void window_reader_kernel(const void *src, const void *scales, void *dst, float *dst_scale, int nkv, int klen,
-                                     int cache_hd, int pitch, int cache_cap, int win_start, int scale_blocks) {
+__global__ void __launch_bounds__(256) window_reader_kernel(const void *src, const void *scales, void *dst, float *dst_scale, int nkv, int klen,
+                                                            int cache_hd, int pitch, int cache_cap, int win_start, int scale_blocks) {
+    // one head per blockIdx.y, 8 elements per thread: 32-bit index arithmetic
     const int groups = cache_hd / 8;
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)nkv * klen * groups) return;
-    const int gcol = (int)(idx % groups);
-    const long t = idx / groups;
-    const int j = (int)(t % klen), h = (int)(t / klen);
-    const size_t sr = (size_t)h * cache_cap + (size_t)((win_start + j) % cache_cap);
+    const unsigned idx = blockIdx.x * 256u + threadIdx.x;
+    const int j = (int)(idx / (unsigned)groups), gcol = (int)(idx - (unsigned)j * groups), h = blockIdx.y + 65535 * blockIdx.z;
+    if (j >= klen || h >= nkv) return;
+    const size_t sr = (size_t)h * cache_cap + ((unsigned)win_start + (unsigned)j) % (unsigned)cache_cap;
     const size_t dr = (size_t)h * pitch + j;
     const int d0 = gcol * 8;
     int q[8];
@@ -217,8 +263,34 @@ int launch_dequant_i8(cudaStream_t st, const void *in_i8, const void *in_scales,
     return check_launch("nomos_kv_dequant_i8");
 }
 
+// Rows of the register kernel (append_rows_kernel): its head dims, int4 rows it may write 4 bytes at a time, no int8 view.
+static bool append_rows_ok(const AppendI4Args &a, int fmt) {
+    if (a.k_q8 || (a.l_hd != 128 && a.l_hd != 256 && a.l_hd != 512)) return false;
+    return fmt == KV_I8 || (a.cache_hd % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.dst_k) | reinterpret_cast<uintptr_t>(a.dst_v)) & 3) == 0);
+}
+template <int FMT>
+static int launch_append_rows(cudaStream_t st, const AppendI4Args &a, const char *who) {
+    cudaLaunchAttribute pdl[1];
+    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks_for(2l * a.n_s * a.nkv, ROWS_PER_BLOCK)); cfg.blockDim = dim3(ROWS_PER_BLOCK * 32); cfg.stream = st;
+    cfg.attrs = pdl; cfg.numAttrs = 1;
+    cudaError_t e = a.l_hd == 128 ? cudaLaunchKernelEx(&cfg, append_rows_kernel<128, FMT>, a)
+                    : a.l_hd == 256 ? cudaLaunchKernelEx(&cfg, append_rows_kernel<256, FMT>, a) : cudaLaunchKernelEx(&cfg, append_rows_kernel<512, FMT>, a);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("%s: %s", who, cudaGetErrorString(e)); return NOMOS_ECUDA; }
+    return NOMOS_OK;
+}
+
 int launch_append_i8(cudaStream_t st, const void *src_k, const void *src_v, void *dst_k, void *dst_v, void *k_scales,
                      void *v_scales, int n_s, int nkv, int l_hd, int l_kvd, int cache_cap, int cache_hd, int base_pos) {
+    AppendI4Args a = {};
+    a.src_k = static_cast<const float *>(src_k); a.src_v = static_cast<const float *>(src_v);
+    a.dst_k = static_cast<uint8_t *>(dst_k); a.dst_v = static_cast<uint8_t *>(dst_v);
+    a.k_scales = k_scales; a.v_scales = v_scales;
+    a.n_s = n_s; a.nkv = nkv; a.l_hd = l_hd; a.l_kvd = l_kvd; a.cache_cap = cache_cap; a.cache_hd = cache_hd; a.base_pos = base_pos;
+    if (append_rows_ok(a, KV_I8)) return launch_append_rows<KV_I8>(st, a, "nomos_kv_append_quant_i8");
     append_i8_kernel<<<blocks_for((long)n_s * nkv, ROWS_PER_BLOCK), ROWS_PER_BLOCK * 32, 0, st>>>(
         static_cast<const float *>(src_k), static_cast<const float *>(src_v), static_cast<int8_t *>(dst_k),
         static_cast<int8_t *>(dst_v), static_cast<float *>(k_scales), static_cast<float *>(v_scales), n_s, nkv, l_hd, l_kvd,
@@ -229,10 +301,15 @@ int launch_append_i8(cudaStream_t st, const void *src_k, const void *src_v, void
 int launch_append_paged_i8(cudaStream_t st, const void *src_k, const void *src_v, void *k_pool, void *v_pool, void *ks_pool,
                            void *vs_pool, const int *block_table, const int *positions, int batch, int nkv, int l_hd, int l_kvd,
                            int max_pages) {
-    append_paged_i8_kernel<<<blocks_for((long)batch * nkv, ROWS_PER_BLOCK), ROWS_PER_BLOCK * 32, 0, st>>>(
-        static_cast<const float *>(src_k), static_cast<const float *>(src_v), static_cast<int8_t *>(k_pool),
-        static_cast<int8_t *>(v_pool), static_cast<float *>(ks_pool), static_cast<float *>(vs_pool), block_table, positions, batch,
-        nkv, l_hd, l_kvd, max_pages);
+    cudaLaunchAttribute pdl[1];
+    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks_for(2l * batch * nkv, ROWS_PER_BLOCK)); cfg.blockDim = dim3(ROWS_PER_BLOCK * 32); cfg.stream = st;
+    cfg.attrs = pdl; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, l_hd == 128 ? append_paged_i8_kernel<true> : append_paged_i8_kernel<false>, static_cast<const float *>(src_k),
+                       static_cast<const float *>(src_v), static_cast<int8_t *>(k_pool), static_cast<int8_t *>(v_pool),
+                       static_cast<float *>(ks_pool), static_cast<float *>(vs_pool), block_table, positions, batch, nkv, l_hd, l_kvd, max_pages);
     return check_launch("nomos_kv_paged_append_quant_i8");
 }
 
@@ -247,23 +324,33 @@ int launch_append_i4(cudaStream_t st, const void *src_k, const void *src_v, void
     a.k_q8_scales = static_cast<float *>(k_q8_scales); a.v_q8_scales = static_cast<float *>(v_q8_scales);
     a.n_s = n_s; a.nkv = nkv; a.l_hd = l_hd; a.l_kvd = l_kvd; a.cache_cap = cache_cap; a.cache_hd = cache_hd;
     a.base_pos = base_pos; a.q8_pitch = q8_pitch; a.scale_blocks = scale_blocks;
+    if (append_rows_ok(a, KV_I4))
+        return scale_blocks > 1 ? launch_append_rows<KV_I4B32>(st, a, "nomos_kv_append_quant_i4") : launch_append_rows<KV_I4>(st, a, "nomos_kv_append_quant_i4");
     append_i4_kernel<<<blocks_for((long)n_s * nkv, ROWS_PER_BLOCK), ROWS_PER_BLOCK * 32, 0, st>>>(a);
     return check_launch("nomos_kv_append_quant_i4");
 }
 
 int launch_window_reader(cudaStream_t st, int mode, const void *src, const void *scales, void *dst, void *dst_scale, int nkv,
                          int klen, int cache_hd, int pitch, int cache_cap, int win_start, int scale_blocks) {
-    const long n = (long)nkv * klen * (cache_hd / 8);
-    const unsigned nb = blocks_for(n, 256);
-    float *ds = static_cast<float *>(dst_scale);
-#define NOMOS_RD(M) window_reader_kernel<M><<<nb, 256, 0, st>>>(src, scales, dst, ds, nkv, klen, cache_hd, pitch, cache_cap, win_start, scale_blocks)
-    switch (mode) {
-        case RD_I8_BF16: NOMOS_RD(RD_I8_BF16); break;
-        case RD_I4_BF16: NOMOS_RD(RD_I4_BF16); break;
-        case RD_I4B32_BF16: NOMOS_RD(RD_I4B32_BF16); break;
-        case RD_I4_Q8: NOMOS_RD(RD_I4_Q8); break;
-        case RD_I4B32_Q8: NOMOS_RD(RD_I4B32_Q8); break;
-        default: set_error("window reader: bad mode %d", mode); return NOMOS_EBADARG;
+    const int groups = cache_hd / 8;
+    if (groups == 0) return NOMOS_OK;
+    const int most = (1 << 30) / groups;                               // rows of a head per launch: 32-bit thread index
+    const int elem = mode <= RD_I4B32_BF16 ? 2 : 1;
+    for (int j0 = 0; j0 < klen; j0 += most) {
+        const int n = std::min(most, klen - j0);
+        const dim3 nb(blocks_for((long)n * groups, 256), (unsigned)std::min(nkv, 65535), (unsigned)((nkv + 65534) / 65535));
+        void *d = static_cast<char *>(dst) + (size_t)j0 * cache_hd * elem;
+        float *ds = dst_scale ? static_cast<float *>(dst_scale) + j0 : nullptr;
+        const int ws = (int)(((long)win_start + j0) % cache_cap);
+#define NOMOS_RD(M) window_reader_kernel<M><<<nb, 256, 0, st>>>(src, scales, d, ds, nkv, n, cache_hd, pitch, cache_cap, ws, scale_blocks)
+        switch (mode) {
+            case RD_I8_BF16: NOMOS_RD(RD_I8_BF16); break;
+            case RD_I4_BF16: NOMOS_RD(RD_I4_BF16); break;
+            case RD_I4B32_BF16: NOMOS_RD(RD_I4B32_BF16); break;
+            case RD_I4_Q8: NOMOS_RD(RD_I4_Q8); break;
+            case RD_I4B32_Q8: NOMOS_RD(RD_I4B32_Q8); break;
+            default: set_error("window reader: bad mode %d", mode); return NOMOS_EBADARG;
+        }
     }
 #undef NOMOS_RD
     return check_launch("nomos_kv_dequant_layer");
