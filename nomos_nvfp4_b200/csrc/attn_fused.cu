@@ -884,11 +884,4 @@ int launch_merge_partials(cudaStream_t st, const float *partials, int G, int row
     return NOMOS_OK;
 }
 
-int launch_merge_partials_log2(cudaStream_t st, const float *partials, int G, int rows, int l_hd, float *out) {
-    merge_kernel<<<rows, 128, 0, st>>>(partials, G, rows, l_hd, out, ET_F32, 0, nullptr);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { set_error("merge launch: %s", cudaGetErrorString(e)); return NOMOS_ECUDA; }
-    return NOMOS_OK;
-}
-
 }  // namespace nomos

@@ -99,8 +99,6 @@ int read_attn_faults(unsigned int *out, bool clear);
 int clear_attn_fault_bits(unsigned int bits);
 // partials [G][rows][l_hd+2] = (o.., m, l) with m in natural-log units (the exported form)
 int launch_merge_partials(cudaStream_t st, const float *partials, int G, int rows, int l_hd, void *out, int out_type);
-// same, m in log2 units (in-library split partials), fp32 output
-int launch_merge_partials_log2(cudaStream_t st, const float *partials, int G, int rows, int l_hd, float *out);
 
 // ---- attn_dense.cu : fp32 / bf16 KV decode + prefix-batched attention
 // K / V / Q producer epilogue (kv_producer.cu): RMSNorm (+ weight), RoPE, quantize-on-write.

@@ -54,3 +54,26 @@ def test_dense_decode_key_counts(dtype, nh, nkv, hd, T):
     kk, vv = (x[:, :T].double().repeat_interleave(nh // nkv, 0) for x in (k, v))
     want = (torch.softmax((q.double()[:, None] * kk).sum(-1), -1)[..., None] * vv).sum(1)
     assert (out.double() - want).abs().max().item() <= 1e-5 * want.square().mean().sqrt().item()
+
+
+@pytest.mark.parametrize("hd,shift", [(128, 0), (512, 0), (256, 8)])
+def test_block32_reader_to_int8_every_code(oracle, hd, shift):
+    """All 16 nibble values under scales from subnormal to large, aligned rows (table kernel) and rows 8 bytes off (general
+    kernel): the same bytes from both, and the reference's arithmetic (multiply, divide, round away) in float32."""
+    rng = np.random.default_rng(hd)
+    nkv, cap, klen, start, nb = 2, 37, 29, 20, hd // 32
+    codes = rng.integers(0, 256, (nkv, cap, hd // 2), dtype=np.uint8)
+    s16 = (2.0 ** rng.uniform(-16, 6, (nkv, cap, nb))).astype(np.float16)
+    q8 = (s16.astype(np.float32).max(-1) * np.float32(7.0) / np.float32(127.0)).astype(np.float32)
+    scales = np.concatenate([s16.view(np.uint8).ravel(), q8.view(np.uint8).ravel()])
+    raw = torch.zeros(codes.size + 64, dtype=torch.uint8, device=DEV)
+    raw[shift:shift + codes.size] = dev(codes.ravel())
+    out, osc = torch.zeros(nkv, klen, hd, dtype=torch.int8, device=DEV), torch.zeros(nkv, klen, device=DEV)
+    ops.gpu_dequant_kv_i4_to_q8_layer(None, raw.data_ptr() + shift, dev(scales), out, osc, nkv, klen, hd, klen, cap, start, nb)
+    torch.cuda.synchronize()
+    slots = (start + np.arange(klen)) % cap
+    nib = np.stack([codes & 15, codes >> 4], -1).reshape(nkv, cap, hd).astype(np.int32)
+    q = ((nib ^ 8) - 8).astype(np.float32)
+    x = (q * np.repeat(s16.astype(np.float32), 32, -1)) / q8[..., None]
+    want = np.clip(np.trunc(x + np.where(x >= 0, np.float32(0.5), np.float32(-0.5)).astype(np.float32)), -127, 127).astype(np.int8)
+    assert np.array_equal(host(out), want[:, slots]) and np.array_equal(host(osc), q8[:, slots])
