@@ -24,14 +24,15 @@
 // weights go back into the SAME columns, hi and lo, as the A operand of PV); "dequant" warps that fetch cache bytes
 // from global memory one operand slot ahead, widen them and fill a ring of K / V slots in the order the tensor core
 // takes them (rows are addressed one by one: rings may wrap); one MMA warp.  head_dim 128: two query tiles per CTA in
-// turn, one tile's softmax under the other's products; wider heads: one query tile with two S buffers, and at 512 two
-// CTAs per query tile that each own 256 output dims.  O stays in tensor memory; it is rescaled in place only when a
+// turn, one tile's softmax under the other's products; wider heads: one query tile with four S buffers, and at 512 two
+// CTAs per query tile that each own 256 output dims.  The order of products and waits is prefill_schedule.h.  O stays in tensor memory; it is rescaled in place only when a
 // row's reference moves, which happens when a chunk exceeds it by more than 2^8 (a handful of times per row).
 // Every wait is an mbarrier wait with a time limit; a wait that runs out raises the CTA's abort flag and bit 1 of the
 // device fault word, every role leaves its loop, tensor memory is freed and the CTA exits.
 #pragma once
 
 #include "attn_tc5_kernel.cuh"
+#include "prefill_schedule.h"
 
 namespace nomos {
 namespace pf {
@@ -66,11 +67,11 @@ struct Cfg {
     // the ring grants only once V of tile i is released (all softmax rows of tile i are then done): ring order
     // K0 K1 V0 K2 V1 ... makes that (nconst - 2) * (KS + VS) >= slots - 1.
     static constexpr int nconst(int slots) { return 2 + (slots - 1 + KS + VS - 1) / (KS + VS); }
-    static constexpr int smem(int slots) { return Q_BYTES + slots * SLOT + nconst(slots) * 3 * KT * 4 + (2 * slots + nconst(slots) + 4 * NQ + 2 * NQ + 1) * 8 + 16; }
+    static constexpr int smem(int slots) { return Q_BYTES + slots * SLOT + nconst(slots) * 3 * KT * 4 + (2 * slots + nconst(slots) + 3 * 4 + 1) * 8 + 16; }
     static constexpr int most_slots() { int n = 2 * KL; while (smem(n + KL) <= SMEM_MAX) n += KL; return n; }
     static constexpr int NSLOT = most_slots(), NCONST = nconst(NSLOT);
     static_assert(NSLOT >= 2 * KL && NSLOT % KL == 0, "a V unit and the K unit behind it; the limbs of a unit side by side");
-    static constexpr int NSB = 2 * NQ;                                 // S buffers: two per query tile
+    static constexpr int NB = s_buffers<NQ>(), NSB = NB * NQ;          // S buffers per query tile, in all
     static constexpr int TMEM_O = 0, TMEM_S = 256;
     static_assert(NQ * DV <= 256 && NSB * KT <= 256, "tensor memory columns");
     static constexpr int NSW = 8 * NQ;                                 // softmax warps: two per 32 TMEM lanes, 16 rows each
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
     const int b = bid % p.batch, qb = p.q_blocks - 1 - bid / p.batch;
 
     // key range of each query tile (whole key tiles), and of the CTA
-    int g_first[NQ], g_last[NQ];                       // tiles of query tile g, relative to the CTA's first (empty: first > last)
+    TileRange range[NQ];                               // tiles of query tile g, relative to the CTA's first (empty: first > last)
     int tile_lo = 0x7fffffff, tile_hi = -1;
 #pragma unroll
     for (int g = 0; g < NQ; ++g) {
@@ -272,16 +273,16 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         const int hi = s_last >= s_first ? min(p.d0 + s_last, p.key_len - 1) : -1;
         const int lo = p.window > 0 ? max(0, p.d0 + s_first - p.window + 1) : 0;
         if (hi >= lo) {
-            g_first[g] = lo / KT; g_last[g] = hi / KT;
-            tile_lo = min(tile_lo, g_first[g]); tile_hi = max(tile_hi, g_last[g]);
+            range[g] = TileRange{lo / KT, hi / KT};
+            tile_lo = min(tile_lo, range[g].first); tile_hi = max(tile_hi, range[g].last);
         } else {
-            g_first[g] = 0x3fffffff; g_last[g] = -1;
+            range[g] = TileRange{0x3fffffff, -1};
         }
     }
     const int n_tiles = tile_hi >= 0 ? tile_hi - tile_lo + 1 : 0;
     if (n_tiles == 0) tile_lo = 0;
 #pragma unroll
-    for (int g = 0; g < NQ; ++g) { g_first[g] -= tile_lo; g_last[g] -= tile_lo; }
+    for (int g = 0; g < NQ; ++g) { range[g].first -= tile_lo; range[g].last -= tile_lo; }
     // (consecutive query tiles have overlapping or adjacent ranges, so every tile of the CTA serves at least one of them;
     // a tile that serves none, possible only with a window shorter than a query tile's span, costs its slots and no products)
 
@@ -324,7 +325,6 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             if (ring == NSLOT) { ring = 0; ring_phase ^= 1u; }
             return ok;
         };
-        auto commit = [&](uint32_t bar) { tc5::umma_commit(bar); };
         // S buffer buf += dims 128 c .. 128 c + 127 of query tile g x the K slots from n on
         auto qk = [&](int g, int buf, int c, int n) {
             const uint32_t d = tmem_base + C::TMEM_S + buf * KT;
@@ -367,61 +367,26 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             tc5::tc_fence_after();
             return ok;
         };
-        bool go = n_tiles > 0 && wait_bar(bar_q_ready, 0);
-        // Ring order K0 K1 V0 K2 V1 ...: with two S buffers per query tile the products of tile i + 1 are done before the
-        // softmax of tile i is, and QK(i + 2) reuses the buffer of PV(i) right behind it (products of one thread run in order).
-        // Buffer and barrier phase follow the query tile's own count of tiles.
-        auto active = [&](int g, int i) { return i >= g_first[g] && i <= g_last[g]; };
-        auto buffer = [&](int g, int i) { return 2 * g + ((i - g_first[g]) & 1); };
-        auto qk_tile = [&](int j) {
-#pragma unroll 1
-            for (int c = 0; c < HD / 128; ++c) {
-                int n;
-                if (!next_unit(n)) return false;
-#pragma unroll
-                for (int g = 0; g < NQ; ++g)
-                    if (active(g, j)) {
-                        qk(g, buffer(g, j), c, n);
-                        if (c == HD / 128 - 1) commit(bar_s_full(buffer(g, j)));
-                    }
-                commit(bar_empty(n));
-            }
-            return true;
-        };
-        go = go && qk_tile(0);
-        if (go && n_tiles > 1) go = qk_tile(1);
-        for (int i = 0; go && i < n_tiles; ++i) {
-            if constexpr (NQ == 2) {
-                // one V unit and one K unit: QK of a query tile goes out behind its PV, before the other tile's weights are waited for
-                int nv, nk = 0;
-                const bool more = i + 2 < n_tiles;
-                if (!(go = next_unit(nv))) break;
-#pragma unroll
-                for (int g = 0; g < NQ; ++g) {
-                    if (go && active(g, i)) {
-                        go = wait_bar(bar_p_full(buffer(g, i)), ((i - g_first[g]) >> 1) & 1);
-                        if (go) { pv(g, buffer(g, i), 0, nv, i == g_first[g]); commit(bar_o_done(buffer(g, i))); }
-                    }
-                    if (g == 1) commit(bar_empty(nv));
-                    if (go && more) {
-                        if (g == 0) go = next_unit(nk);
-                        if (go && active(g, i + 2)) { qk(g, buffer(g, i + 2), 0, nk); commit(bar_s_full(buffer(g, i + 2))); }
-                    }
-                }
-                if (go && more) commit(bar_empty(nk));
-            } else {
-                if (!(go = wait_bar(bar_p_full(buffer(0, i)), (i >> 1) & 1))) break;
-#pragma unroll 1
-                for (int c = 0; c < DV / 128; ++c) {
-                    int n;
-                    if (!(go = next_unit(n))) break;
-                    pv(0, buffer(0, i), c, n, i == 0);
-                    commit(bar_empty(n));
-                }
-                if (!go) break;
-                commit(bar_o_done(buffer(0, i)));
-                if (i + 2 < n_tiles) go = qk_tile(i + 2);
-            }
+        if (n_tiles > 0 && wait_bar(bar_q_ready, 0)) {
+            struct Ops {
+                decltype(next_unit) &next;
+                decltype(wait_bar) &wait;
+                decltype(qk) &qk_;
+                decltype(pv) &pv_;
+                decltype(bar_empty) &empty;
+                decltype(bar_s_full) &s_full;
+                decltype(bar_p_full) &p_full;
+                decltype(bar_o_done) &od;
+                __device__ __forceinline__ bool next_unit(int &slot) { return next(slot); }
+                __device__ __forceinline__ void release(int slot) { tc5::umma_commit(empty(slot)); }
+                __device__ __forceinline__ bool weights(int buf, int parity) { return wait(p_full(buf), parity); }
+                __device__ __forceinline__ bool product(int buf, int parity) { return wait(od(buf), parity); }
+                __device__ __forceinline__ void qk(int g, int buf, int c, int slot) { qk_(g, buf, c, slot); }
+                __device__ __forceinline__ void s_done(int buf) { tc5::umma_commit(s_full(buf)); }
+                __device__ __forceinline__ void pv(int g, int buf, int c, int slot, bool first) { pv_(g, buf, c, slot, first); }
+                __device__ __forceinline__ void o_done(int buf) { tc5::umma_commit(od(buf)); }
+            } ops{next_unit, wait_bar, qk, pv, bar_empty, bar_s_full, bar_p_full, bar_o_done};
+            walk_products<NQ, HD / 128, DV / 128>(n_tiles, range, ops);
         }
         }
         __syncwarp();
@@ -448,27 +413,13 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         int soff[NCH];
 #pragma unroll
         for (int e = 0; e < NCH; ++e) soff[e] = op_off(prow, NCH * ppc + e, C::BLOCK);
-        // unit i of the ring order K0 K1 V0 K2 V1 ...: V tile or K tile, and which 128 dims
-        constexpr int KU = HD / 128, VU = DV / 128;
-        struct Unit { int tile, v, c; };
-        auto unit_at = [&](int i) {
-            const int lead = KU * min(n_tiles, 2);
-            if (i < lead) return Unit{i / KU, 0, i % KU};
-            i -= lead;
-            const int body = (KU + VU) * max(0, n_tiles - 2);
-            if (i < body) {
-                const int q = i / (KU + VU), r = i % (KU + VU);
-                return r < VU ? Unit{q, 1, r} : Unit{q + 2, 0, r - VU};
-            }
-            i -= body;
-            return Unit{max(0, n_tiles - 2) + i / VU, 1, i % VU};
-        };
+        auto unit_at = [&](int i) { return ring_unit<HD / 128, DV / 128>(i, n_tiles); };
         constexpr int NBW = C::NBW, NP = C::NP, TEAMS = C::TEAMS;
         constexpr int NSC = FMT == KV_I4B32 ? NP : 1, NCW = FMT == KV_I4B32 ? NBW : 1;
         // cache bytes of the team's next unit; with the first K unit of a tile the scales of key t of the tile
         uint4 x[NP];
         uint32_t sc[NSC], ckw[NCW], cvw[NCW];
-        auto fetch = [&](Unit u) {
+        auto fetch = [&](RingUnit u) {
             const uint8_t *base = u.v ? gv : gk;
             const int key0 = (tile_lo + u.tile) * KT;
             const int dim0 = (u.v ? dpart * DV : 0) + u.c * 128;       // first dim of the slot
@@ -518,7 +469,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             if (lane == 0) tc5::mbar_arrive(bar_const(tile % NCONST));
         };
         static_assert(KT == 64, "a team's 64 threads take one key each");
-        auto convert = [&](Unit u, int slot) {
+        auto convert = [&](RingUnit u, int slot) {
             uint8_t *s0 = sm + C::OFF_RING + slot * C::SLOT;
             uint8_t *s1 = s0 + (KL - 1) * C::SLOT;
             const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (u.tile % NCONST) * 3 * KT;
@@ -561,7 +512,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         const int n_units = n_tiles * ((HD + DV) / 128);
         auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, p.fault)) != 0; };
         // this team's units are team, team + TEAMS, ...; its next one is on the way while the other teams' are converted
-        Unit u = unit_at(team);
+        RingUnit u = unit_at(team);
         if (team < n_units) fetch(u);
         for (int i = team; i < n_units; i += TEAMS) {
             const int n = i * KL, lap = n / NSLOT, slot = n - lap * NSLOT;
@@ -681,15 +632,15 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             if (lane == 0) tc5::mbar_arrive(bar_q_ready);
         }
         bool alive = true;
-        const int first = NQ == 2 && g == 1 ? g_first[NQ - 1] : g_first[0], last = NQ == 2 && g == 1 ? g_last[NQ - 1] : g_last[0];
+        const int first = NQ == 2 && g == 1 ? range[NQ - 1].first : range[0].first, last = NQ == 2 && g == 1 ? range[NQ - 1].last : range[0].last;
         for (int i = max(first, 0); alive && i <= last; ++i) {
             const int it = i - first;                                  // this row's tiles so far
-            const int buf = 2 * g + (it & 1);
+            const int buf = C::NB * g + it % C::NB;
             const uint32_t ts = tmem_lane + C::TMEM_S + buf * KT;
             const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (i % NCONST) * 3 * KT;
             // (the constants were stored before the K slots of the tile: this wait only orders the reads; it may not come
             // first, a query tile whose range starts late would meet an older phase of the barrier)
-            if (!wait_warp(bar_s_full(buf), (it >> 1) & 1)) { alive = false; break; }
+            if (!wait_warp(bar_s_full(buf), (it / C::NB) & 1)) { alive = false; break; }
             if (!wait_warp(bar_const(i % NCONST), (i / NCONST) & 1)) { alive = false; break; }
             tc5::tc_fence_after();
             const int t0 = (tile_lo + i) * KT;
@@ -748,7 +699,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
                     l[q].x *= alpha[q]; l[q].y *= alpha[q];
                 }
                 if (it > 0) {
-                    if (!wait_warp(bar_o_done(2 * g + ((it - 1) & 1)), ((it - 1) >> 1) & 1)) { alive = false; break; }
+                    if (!wait_warp(bar_o_done(C::NB * g + (it - 1) % C::NB), ((it - 1) / C::NB) & 1)) { alive = false; break; }
                     tc5::tc_fence_after();
 #pragma unroll 1
                     for (int c = 0; c < DV / 32; ++c) {
@@ -788,8 +739,8 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         }
         // ---- output: O / l (rows without any key are exact zeros, lib/batched_attn_gpu.mojo:329-409)
         const int mine = last >= max(first, 0) ? last - first + 1 : 0;
-        // (the barrier's phase before that is known to be over: S of the last tile was issued behind that PV)
-        if (alive && mine > 0) alive = wait_warp(bar_o_done(2 * g + ((mine - 1) & 1)), ((mine - 1) >> 1) & 1);
+        // (the barrier's phase before that is known to be over: S of the last tile was issued once that PV was done)
+        if (alive && mine > 0) alive = wait_warp(bar_o_done(C::NB * g + (mine - 1) % C::NB), ((mine - 1) / C::NB) & 1);
         if (alive) {
             tc5::tc_fence_after();
             float inv[2];
