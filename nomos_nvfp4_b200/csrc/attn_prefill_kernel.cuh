@@ -226,14 +226,72 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-// Block-32 rows: power of two that takes the row's largest block scale to [2^11, 2^12) (times any code it stays below
-// the fp16 maximum, and the low limb of a block 2^-10 of the largest still has all its bits).
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// Block-32 rows: power of two that takes the row's largest finite block scale to [2^11, 2^12) (times any code it stays
+// below the fp16 maximum, and the low limb of a block 2^-10 of the largest still has all its bits).  `nonfinite`: some
+// block's scale is infinite or NaN.
 template <int NBW>
-__device__ __forceinline__ int b32_shift(const uint32_t (&w)[NBW]) {
-    uint32_t mx = 0;
+__device__ __forceinline__ int b32_shift(const uint32_t (&w)[NBW], bool &nonfinite) {
+    uint32_t m = 0, over = 0;                                          // largest exponent + 1 of either half; infinities and NaNs run over
 #pragma unroll
-    for (int i = 0; i < NBW; ++i) mx = max(mx, max(w[i] & 0x7fffu, (w[i] >> 16) & 0x7fffu));
-    return 26 - max(1, (int)(mx >> 10));
+    for (int i = 0; i < NBW; ++i) {
+        const uint32_t e = (w[i] & 0x7fff7fffu) + 0x04000400u;
+        m = max_u16x2(m, e & 0x7fff7fffu);
+        over |= e & 0x80008000u;
+    }
+    nonfinite = over != 0;
+    return 27 - max(2, (int)(max(m & 0xffffu, m >> 16) >> 10));
+}
+// Block-32 caches whose value scales overflowed fp16 (the codec stores infinity for blocks beyond 7 x 65504): adds such
+// blocks to the output rows whose keys include them; any weight leaves code x infinity what it is.  Called by the softmax
+// warps on the rows and dims each of their threads wrote.  Rare: one key at a time, out of line, and the CTA's place worked
+// out again (in line, its registers cost the loops 84.9 -> 87.5 us for 2048 positions at head_dim 128; so 85.7).
+template <int HD, int DV, int NQ>
+__device__ __noinline__ void add_nonfinite_values(const PParams &p) {
+    int bid;
+    asm volatile("mov.u32 %0, %%ctaid.x;\n" : "=r"(bid));
+    const int dpart = bid % (HD / DV);
+    bid /= HD / DV;
+    const int kvh = bid % p.nkv;
+    bid /= p.nkv;
+    const int b = bid % p.batch, tile = (p.q_blocks - 1 - bid / p.batch) * NQ + (NQ == 2 ? threadIdx.x >> 8 : 0);
+    const int lane = threadIdx.x & 31, first_row = 32 * ((threadIdx.x >> 5) & 3) + 16 * ((threadIdx.x >> 7) & 1) + (lane >> 2);
+#pragma unroll 1
+    for (int row = first_row; row < first_row + 16; row += 8) {
+        const int pos = tile * p.pos_per_tile + row / p.kvg;
+        if (row >= p.pos_per_tile * p.kvg || pos >= p.S) continue;
+        const int hi = min(p.d0 + pos, p.key_len - 1), lo = p.window > 0 ? max(0, p.d0 + pos - p.window + 1) : 0;
+        const long at = b * p.out_batch_stride + ((long)pos * p.nh + kvh * p.kvg + row % p.kvg) * HD + dpart * DV + 2 * (lane & 3);
+#pragma unroll 1
+        for (int key = lo; key <= hi; ++key) {
+            int slot = p.row0 + key;
+            if (slot >= p.cache_cap) slot -= p.cache_cap;
+            const size_t cr = (size_t)kvh * p.cache_cap + slot;
+            const __half *scales = reinterpret_cast<const __half *>(p.v_scales + b * p.scale_batch_stride) + cr * (HD / 32) + dpart * (DV / 32);
+            const uint8_t *codes = p.v_cache + b * p.kv_batch_stride + cr * p.row_bytes + dpart * (DV / 2) + (lane & 3);
+#pragma unroll 1
+            for (int c = 0; c < DV / 32; ++c) {
+                const float sf = __half2float(scales[c]);
+                if (isfinite(sf)) continue;
+                for (int e = 0; e < 4; ++e) {
+                    const int byte = codes[16 * c + 4 * e];
+                    const float x = (float)nib_sext(byte & 15) * sf, y = (float)nib_sext(byte >> 4) * sf;
+                    const long d = at + 32 * c + 8 * e;
+                    if (p.out_type == ET_BF16) {
+                        __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(p.out) + d);
+                        *o = __floats2bfloat162_rn(__low2float(*o) + x, __high2float(*o) + y);
+                    } else {
+                        float2 *o = reinterpret_cast<float2 *>(reinterpret_cast<float *>(p.out) + d);
+                        *o = make_float2(o->x + x, o->y + y);
+                    }
+                }
+            }
+        }
+    }
 }
 
 template <int HD, int FMT, int QL>
@@ -245,6 +303,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
     const uint32_t sm_u32 = smem_u32(sm);
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(sm + C::OFF_MISC);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + C::OFF_MISC + 4);
+    volatile int *v_nonfinite = reinterpret_cast<volatile int *>(sm + C::OFF_MISC + 8);       // block-32: some value block's scale is infinite or NaN
     const uint32_t bar0 = sm_u32 + C::OFF_BAR;
     auto bar_full = [&](int s) { return bar0 + 8 * s; };                          // dequant warps -> MMA
     auto bar_empty = [&](int s) { return bar0 + 8 * (NSLOT + s); };               // commit after the slot's last product -> dequant
@@ -288,6 +347,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
+        *v_nonfinite = 0;
         for (int s = 0; s < NSLOT; ++s) { fused::mbar_init(bar_full(s), 2); fused::mbar_init(bar_empty(s), 1); }
         for (int i = 0; i < NCONST; ++i) fused::mbar_init(bar_const(i), 2);
         for (int i = 0; i < NSB; ++i) { fused::mbar_init(bar_s_full(i), 1); fused::mbar_init(bar_p_full(i), 8); fused::mbar_init(bar_o_done(i), 1); }
@@ -455,7 +515,9 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         auto store_const = [&](int tile) {                 // per-key constants of the tile (block-32: with the shifts the conversion reads back)
             float *cc = reinterpret_cast<float *>(sm + C::OFF_CONST) + (tile % NCONST) * 3 * KT;
             if constexpr (FMT == KV_I4B32) {
-                const int sk = b32_shift(ckw), sv = b32_shift(cvw);
+                bool k_bad, v_bad;
+                const int sk = b32_shift(ckw, k_bad), sv = b32_shift(cvw, v_bad);
+                if (v_bad) *v_nonfinite = 1;
                 cc[t] = pow2i(-sk);
                 cc[KT + t] = (float)(-sv);
                 cc[2 * KT + t] = pow2i(sv);
@@ -473,6 +535,10 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             uint8_t *s0 = sm + C::OFF_RING + slot * C::SLOT;
             uint8_t *s1 = s0 + (KL - 1) * C::SLOT;
             const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (u.tile % NCONST) * 3 * KT;
+            // zero weight x infinity is not zero: rows that may not see a key would be lost to its value, so infinities and
+            // NaNs among V's block scales become finite here and reach the rows that do see them in add_nonfinite_values.
+            // (A K row's leave through the select that masks the logits.)
+            const float most = u.v ? 4096.0f : CUDART_INF_F;
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 const int row = prow + k * RSTEP, koff = k * RSTEP * 128;
@@ -489,7 +555,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
                         const uint32_t bits = (ppc & 1) ? sc[k] >> 16 : sc[k] & 0xffffu;        // (slots start at even blocks)
                         // the row's power of two: 1 / logit factor for K, 1 / value scale for V
                         const float up = u.v ? cc[2 * KT + row] : __uint_as_float(0x7f000000u - __float_as_uint(cc[row]));
-                        const float sf = __half2float(__ushort_as_half((unsigned short)bits)) * up;
+                        const float sf = fmaxf(fminf(__half2float(__ushort_as_half((unsigned short)bits)) * up, most), -most);
                         const float sh = __uint_as_float(__float_as_uint(sf) & 0xfffe0000u);       // top 7 significant bits
                         hi2 = pack_f16x2(sh, sh);
                         lo2 = pack_f16x2(sf - sh, sf - sh);
@@ -785,6 +851,8 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
     tc5::tc_fence_before();
     __syncthreads();
     if (warp == C::W_MMA) tc5::tmem_dealloc(tmem_base, 512);
+    if (FMT == KV_I4B32 && warp < C::NSW && *v_nonfinite && !*abort_flag)
+        add_nonfinite_values<HD, DV, NQ>(p);
 }
 
 }  // namespace pf

@@ -104,6 +104,44 @@ def test_a_row_of_infinities_stays_alone(oracle):
     assert np.array_equal(got[0][keep], clean[0][keep])
 
 
+@pytest.mark.parametrize("q_type", [ops.F32, ops.BF16])
+@pytest.mark.parametrize("hd", [128, 256, 512])
+def test_an_infinite_value_block_reaches_only_the_rows_that_see_it(oracle, hd, q_type):
+    """A block of one V row overflows its fp16 scale (or is infinite from the start): rows in front of the key and rows
+    whose window has passed it are bit for bit what they are without it, the others lose that block's dims and no more."""
+    if not served(hd, q_type):
+        pytest.skip("fp32 queries of 512-wide heads run as row groups")
+    rng = np.random.default_rng(hd + 5)
+    nkv, kvg, S, T, window, key, blk = 2, 2, 150, 200, 40, 101, hd // 32 - 2
+    k, v = bf16_normal(rng, (T, nkv, hd)), bf16_normal(rng, (T, nkv, hd))
+    q, scale = bf16_normal(rng, (S, nkv * kvg, hd)), 1.0 / np.sqrt(hd)
+    outs = []
+    for bad in (False, True):
+        c = KVCache("i4b32", nkv, T, hd)
+        if bad:
+            v[key, 0, 32 * blk:32 * blk + 32] *= np.float32(1e7)
+            v[key, 1, 32 * blk + 3] = np.inf
+        c.append(k, v, 0)
+        if bad:                                        # codes of both signs under the infinite scale: infinities, not only NaNs
+            c.v[0, key, 16 * blk:16 * blk + 4] = [0x71, 0xf0, 0x08, 0x9a]
+        got, choice = run_fused(c, q, S=S, klen=T, window=window, scale=scale, q_type=q_type, out_type=q_type, flags=ops.TCGEN05_ALWAYS)
+        assert choice == 2
+        outs.append(got[0])
+    rows = np.arange(S) + T - S
+    sees = (rows >= key) & (rows < key + window)
+    assert np.array_equal(outs[1][~sees], outs[0][~sees])
+    want = oracle.attn_exact(q, c.k, c.v, c.ks, c.vs, c.kv_fmt, nkv * kvg, nkv, hd, hd, T, S=S, window=window, query_base_pos=T - S, softmax_scale=scale)
+    dims = np.zeros(hd, bool)
+    dims[32 * blk:32 * blk + 32] = True
+    assert np.array_equal(outs[1][sees][..., dims], want[sees][..., dims], equal_nan=True) and not np.isfinite(want[sees][..., dims]).any()
+    for r in np.flatnonzero(sees):
+        if q_type == ops.BF16:
+            assert np.all(np.abs(outs[1][r][:, ~dims] - want[r][:, ~dims]) <= np.abs(want[r][:, ~dims]) * 2.0 ** -8 + TOL)
+        else:
+            ok, rel = within(outs[1][r][:, ~dims], want[r][:, ~dims], TOL)
+            assert ok, f"row {r}: {rel:.2e} x RMS"
+
+
 @pytest.mark.parametrize("hd,nh,nkv,fmt,S,klen,window,choice", [
     (256, 32, 16, "i8", 13, 2048, 0, 0), (256, 32, 16, "i8", 1024, 2048, 1024, 2), (256, 32, 16, "i4b32", 24, 16384, 0, 0),
     (512, 32, 4, "i4b32", 509, 4093, 0, 2), (512, 32, 4, "i8", 16, 16384, 0, 0), (128, 32, 16, "i4", 2048, 2048, 0, 2),
