@@ -231,20 +231,25 @@ __device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
     asm("max.u16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-// Block-32 rows: power of two that takes the row's largest finite block scale to [2^11, 2^12) (times any code it stays
-// below the fp16 maximum, and the low limb of a block 2^-10 of the largest still has all its bits).  `nonfinite`: some
-// block's scale is infinite or NaN.
+// Block-32 rows: the power of two that a row's scales are multiplied with before they go into an fp16 operand.  Times any
+// code the largest stays below the fp16 maximum if the scale does not exceed 2^12, and a scale of 2^-14 still has all its
+// bits in the two limbs.  K rows: the largest finite scale to [2^11, 2^12).  V rows: the mean of the exponents to 2^-1,
+// further down only for a scale beyond 2^12 times that: what is taken out of the operand rides in the row's weights, and
+// with the largest scale there one outlier block left the other blocks' weights 2^-25 of ITS size (scales 2^16 apart:
+// errors of 1e-2).  `nonfinite`: some block's scale is infinite or NaN (not counted).
 template <int NBW>
-__device__ __forceinline__ int b32_shift(const uint32_t (&w)[NBW], bool &nonfinite) {
-    uint32_t m = 0, over = 0;                                          // largest exponent + 1 of either half; infinities and NaNs run over
+__device__ __forceinline__ int b32_shift(const uint32_t (&w)[NBW], bool v, bool &nonfinite) {
+    uint32_t m = 0, sum = 0, over = 0;                                 // of exponents + 1, both halves of a word; infinities and NaNs run over
 #pragma unroll
     for (int i = 0; i < NBW; ++i) {
-        const uint32_t e = (w[i] & 0x7fff7fffu) + 0x04000400u;
-        m = max_u16x2(m, e & 0x7fff7fffu);
-        over |= e & 0x80008000u;
+        const uint32_t x = (w[i] & 0x7fff7fffu) + 0x04000400u, e = (x >> 10) & 0x001f001fu;
+        m = max_u16x2(m, e);
+        sum += e;
+        over |= x & 0x80008000u;
     }
     nonfinite = over != 0;
-    return 27 - max(2, (int)(max(m & 0xffffu, m >> 16) >> 10));
+    const int most = 27 - max(2, (int)max(m & 0xffffu, m >> 16));
+    return v ? min(most, 15 - (int)(((sum & 0xffffu) + (sum >> 16)) / (2 * NBW))) : most;
 }
 // Block-32 caches whose value scales overflowed fp16 (the codec stores infinity for blocks beyond 7 x 65504): adds such
 // blocks to the output rows whose keys include them; any weight leaves code x infinity what it is.  Called by the softmax
@@ -516,7 +521,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             float *cc = reinterpret_cast<float *>(sm + C::OFF_CONST) + (tile % NCONST) * 3 * KT;
             if constexpr (FMT == KV_I4B32) {
                 bool k_bad, v_bad;
-                const int sk = b32_shift(ckw, k_bad), sv = b32_shift(cvw, v_bad);
+                const int sk = b32_shift(ckw, false, k_bad), sv = b32_shift(cvw, true, v_bad);
                 if (v_bad) *v_nonfinite = 1;
                 cc[t] = pow2i(-sk);
                 cc[KT + t] = (float)(-sv);

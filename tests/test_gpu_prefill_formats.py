@@ -142,6 +142,28 @@ def test_an_infinite_value_block_reaches_only_the_rows_that_see_it(oracle, hd, q
             assert ok, f"row {r}: {rel:.2e} x RMS"
 
 
+@pytest.mark.parametrize("hd", [128, 256, 512])
+def test_an_outlier_value_block_costs_the_other_blocks_nothing(oracle, hd):
+    """One block of one V row is 2^16 times the others (its scale near the largest fp16): the row's other dims, where it adds
+    nothing unusual, keep the accuracy of ordinary rows."""
+    rng = np.random.default_rng(hd + 6)
+    nkv, kvg, S, T, key, blk = 2, 2, 100, 300, 60, 1
+    c = KVCache("i4b32", nkv, T, hd)
+    k, v = bf16_normal(rng, (T, nkv, hd)), bf16_normal(rng, (T, nkv, hd))
+    v[key, :, 32 * blk:32 * blk + 32] *= np.float32(2.0 ** 16)
+    c.append(k, v, 0)
+    q, scale = bf16_normal(rng, (S, nkv * kvg, hd)), 1.0 / np.sqrt(hd)
+    got, choice = run_fused(c, q, S=S, klen=T, scale=scale, q_type=ops.BF16, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    want = oracle.attn_exact(q, c.k, c.v, c.ks, c.vs, c.kv_fmt, nkv * kvg, nkv, hd, hd, T, S=S, query_base_pos=T - S, softmax_scale=scale)
+    dims = np.zeros(hd, bool)
+    dims[32 * blk:32 * blk + 32] = True
+    for part in (dims, ~dims):
+        for r in range(S):
+            ok, rel = within(got[0][r][:, part], want[r][:, part], TOL)
+            assert ok, f"row {r}: {rel:.2e} x RMS"
+
+
 @pytest.mark.parametrize("hd,nh,nkv,fmt,S,klen,window,choice", [
     (256, 32, 16, "i8", 13, 2048, 0, 0), (256, 32, 16, "i8", 1024, 2048, 1024, 2), (256, 32, 16, "i4b32", 24, 16384, 0, 0),
     (512, 32, 4, "i4b32", 509, 4093, 0, 2), (512, 32, 4, "i8", 16, 16384, 0, 0), (128, 32, 16, "i4", 2048, 2048, 0, 2),
