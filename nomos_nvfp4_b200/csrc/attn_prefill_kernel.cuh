@@ -43,7 +43,7 @@ using tc5::wait_or_abort;
 constexpr int MR = 128;                       // query rows per tile = M of the MMAs
 constexpr float M_INIT = -1.0e30f;
 constexpr float LAZY = 8.0f;                  // base-2 slack before a row's running reference is moved
-constexpr float VS_MIN = 1.0e-30f;            // value scales below this count as this (codecs write none)
+constexpr float VS_MIN = 1.0e-30f;            // value scales of smaller size count as this (1 / scale stays finite)
 constexpr int KT = 64;                        // keys per tile
 constexpr int SMEM_MAX = 232448;              // shared memory a CTA may ask for
 
@@ -67,7 +67,8 @@ struct Cfg {
     // the ring grants only once V of tile i is released (all softmax rows of tile i are then done): ring order
     // K0 K1 V0 K2 V1 ... makes that (nconst - 2) * (KS + VS) >= slots - 1.
     static constexpr int nconst(int slots) { return 2 + (slots - 1 + KS + VS - 1) / (KS + VS); }
-    static constexpr int smem(int slots) { return Q_BYTES + slots * SLOT + nconst(slots) * 3 * KT * 4 + (2 * slots + nconst(slots) + 3 * 4 + 1) * 8 + 16; }
+    static constexpr int CONST_BYTES = 3 * KT * 4 + 8;                 // per-key constants of a tile, and a bit per key
+    static constexpr int smem(int slots) { return Q_BYTES + slots * SLOT + nconst(slots) * CONST_BYTES + (2 * slots + nconst(slots) + 3 * 4 + 1) * 8 + 16; }
     static constexpr int most_slots() { int n = 2 * KL; while (smem(n + KL) <= SMEM_MAX) n += KL; return n; }
     static constexpr int NSLOT = most_slots(), NCONST = nconst(NSLOT);
     static_assert(NSLOT >= 2 * KL && NSLOT % KL == 0, "a V unit and the K unit behind it; the limbs of a unit side by side");
@@ -84,8 +85,9 @@ struct Cfg {
     static constexpr int NTHREADS = 32 * (NSW + ND + 1);
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_RING = Q_BYTES;
-    static constexpr int OFF_CONST = OFF_RING + NSLOT * SLOT;          // [NCONST][3][KT] fp32: logit factor, log2(vscale), 1 / vscale
-    static constexpr int OFF_BAR = OFF_CONST + NCONST * 3 * KT * 4;
+    // [NCONST]: fp32 [KT] each of logit factor, log2(vs) and 1 / vs, vs = |value scale|; then the keys with a negative one
+    static constexpr int OFF_CONST = OFF_RING + NSLOT * SLOT;
+    static constexpr int OFF_BAR = OFF_CONST + NCONST * CONST_BYTES;
     static constexpr int NBAR = 2 * NSLOT + NCONST + 3 * NSB + 1;
     static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;
     static constexpr int SMEM_BYTES = OFF_MISC + 16;                   // (no static shared memory: the dynamic part starts 1024-byte aligned)
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             }
         };
         auto store_const = [&](int tile) {                 // per-key constants of the tile (block-32: with the shifts the conversion reads back)
-            float *cc = reinterpret_cast<float *>(sm + C::OFF_CONST) + (tile % NCONST) * 3 * KT;
+            float *cc = reinterpret_cast<float *>(sm + C::OFF_CONST + (tile % NCONST) * C::CONST_BYTES);
             if constexpr (FMT == KV_I4B32) {
                 bool k_bad, v_bad;
                 const int sk = b32_shift(ckw, false, k_bad), sv = b32_shift(cvw, true, v_bad);
@@ -527,10 +529,13 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
                 cc[KT + t] = (float)(-sv);
                 cc[2 * KT + t] = pow2i(sv);
             } else {
-                const float vs = fmaxf(__uint_as_float(cvw[0]), VS_MIN);
+                // (a NaN goes in with the logit: masked keys lose it in the mask's select)
+                const float v = __uint_as_float(cvw[0]), vs = fmaxf(fabsf(v), VS_MIN);
                 cc[t] = __uint_as_float(ckw[0]);
-                cc[KT + t] = lg2f(vs);
+                cc[KT + t] = v == v ? lg2f(vs) : v;
                 cc[2 * KT + t] = 1.0f / vs;
+                const uint32_t neg = __ballot_sync(0xffffffffu, v < 0.0f);
+                if (lane == 0) reinterpret_cast<uint32_t *>(cc + 3 * KT)[t >> 5] = neg;
             }
             __syncwarp();
             if (lane == 0) tc5::mbar_arrive(bar_const(tile % NCONST));
@@ -539,7 +544,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
         auto convert = [&](RingUnit u, int slot) {
             uint8_t *s0 = sm + C::OFF_RING + slot * C::SLOT;
             uint8_t *s1 = s0 + (KL - 1) * C::SLOT;
-            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (u.tile % NCONST) * 3 * KT;
+            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST + (u.tile % NCONST) * C::CONST_BYTES);
             // zero weight x infinity is not zero: rows that may not see a key would be lost to its value, so infinities and
             // NaNs among V's block scales become finite here and reach the rows that do see them in add_nonfinite_values.
             // (A K row's leave through the select that masks the logits.)
@@ -708,7 +713,7 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
             const int it = i - first;                                  // this row's tiles so far
             const int buf = C::NB * g + it % C::NB;
             const uint32_t ts = tmem_lane + C::TMEM_S + buf * KT;
-            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST) + (i % NCONST) * 3 * KT;
+            const float *cc = reinterpret_cast<const float *>(sm + C::OFF_CONST + (i % NCONST) * C::CONST_BYTES);
             // (the constants were stored before the K slots of the tile: this wait only orders the reads; it may not come
             // first, a query tile whose range starts late would meet an older phase of the barrier)
             if (!wait_warp(bar_s_full(buf), (it / C::NB) & 1)) { alive = false; break; }
@@ -799,6 +804,19 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_ke
                     ph[2 * e + q] = *reinterpret_cast<const uint32_t *>(&hh);
                     w = fma2(F2{__low2float(hh), __high2float(hh)}, minus1, w);
                     pl[2 * e + q] = pack_f16x2(w.x, w.y);
+                }
+            }
+            if constexpr (FMT != KV_I4B32) {
+                // negative value scales (no codec here writes one): the sign goes on the weights, past the denominator
+                const uint2 neg = *reinterpret_cast<const uint2 *>(cc + 3 * KT);
+                if ((neg.x | neg.y) != 0) {
+#pragma unroll
+                    for (int e = 0; e < KT / 8; ++e) {
+                        const uint32_t two = (e < 4 ? neg.x : neg.y) >> (8 * (e & 3) + 2 * (lane & 3));
+                        const uint32_t sign = ((two & 1u) << 15) | ((two & 2u) << 30);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) { ph[2 * e + q] ^= sign; pl[2 * e + q] ^= sign; }
+                    }
                 }
             }
             tmem_st_pairs32(ts, ph);

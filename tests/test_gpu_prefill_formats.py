@@ -164,6 +164,29 @@ def test_an_outlier_value_block_costs_the_other_blocks_nothing(oracle, hd):
             assert ok, f"row {r}: {rel:.2e} x RMS"
 
 
+@pytest.mark.parametrize("hd,fmt", [(128, "i8"), (128, "i4"), (256, "i8"), (512, "i4")])
+def test_negative_and_nan_value_scales(oracle, hd, fmt):
+    """Row scales no codec here writes: negative ones multiply through like any other, a NaN one makes the rows that see its
+    key NaN and no others."""
+    rng = np.random.default_rng(hd + 7)
+    nkv, kvg, S, T, key = 2, 2, 90, 260, 211
+    c = build_cache(fmt, rng, T, nkv, hd)
+    vs = c.vs.view(np.float32).reshape(nkv, T)
+    vs *= np.where(rng.random((nkv, T)) < 0.3, np.float32(-1), np.float32(1))
+    q, scale = bf16_normal(rng, (S, nkv * kvg, hd)), 1.0 / np.sqrt(hd)
+    for nan in (False, True):
+        if nan:
+            vs[1, key] = np.nan
+        got, choice = run_fused(c, q, S=S, klen=T, scale=scale, q_type=ops.BF16, flags=ops.TCGEN05_ALWAYS)
+        assert choice == 2
+        want = oracle.attn_exact(q, c.k, c.v, c.ks, c.vs, c.kv_fmt, nkv * kvg, nkv, hd, hd, T, S=S, query_base_pos=T - S, softmax_scale=scale)
+        lost = np.isnan(want)
+        assert lost.any() == nan and np.array_equal(np.isnan(got[0]), lost)
+        for r in range(S):
+            ok, rel = within(got[0][r][~lost[r]], want[r][~lost[r]], TOL)
+            assert ok, f"row {r}: {rel:.2e} x RMS"
+
+
 @pytest.mark.parametrize("hd,nh,nkv,fmt,S,klen,window,choice", [
     (256, 32, 16, "i8", 13, 2048, 0, 0), (256, 32, 16, "i8", 1024, 2048, 1024, 2), (256, 32, 16, "i4b32", 24, 16384, 0, 0),
     (512, 32, 4, "i4b32", 509, 4093, 0, 2), (512, 32, 4, "i8", 16, 16384, 0, 0), (128, 32, 16, "i4", 2048, 2048, 0, 2),
