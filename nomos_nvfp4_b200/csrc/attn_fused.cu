@@ -752,12 +752,14 @@ static int dispatch_mma(cudaStream_t st, const AttnArgs &a, bool q, long *ws) {
 // few query rows against a long cache leave the chip idle.  Constants from launches back to back on one box, 512 / 2048 /
 // 16384 keys x 13 to 256 rows (row groups / query-major, us): 32q/16kv x 256 int8, bf16 queries, 2048 keys: 13 rows 21 / 58,
 // 48 rows 54 / 57, 64 rows 53 / 57, 96 rows 78 / 58, 256 rows 184 / 57; 512 keys: 13 rows 13 / 21, 256 rows 74 / 22;
-// 32q/4kv x 512 block-32, 2048 keys: 64 rows 114 / 132, 96 rows 169 / 132, 256 rows 393 / 134.
+// 32q/4kv x 512 block-32, 2048 keys: 64 rows 114 / 132, 96 rows 169 / 132, 256 rows 393 / 134.  int8 x 128, positions x keys,
+// bf16: 32q/16kv 24 x 4096 21 / 81, 24 x 16384 49 / 294, 64 x 4096 46 / 82, 128 x 4096 92 / 107, 256 x 4096 141 / 107,
+// 512 x 2048 126 / 59; 8q/4kv 64 x 16384 37 / 293, 512 x 2048 58 / 59, 1024 x 2048 76 / 59.
 static bool prefers_row_groups(const AttnArgs &a) {
     const bool b32 = a.kv_fmt == KV_I4B32, f32 = a.q_type == ET_F32;
     const double keys = a.window > 0 ? std::min<long>(a.klen, (long)a.window + a.S - 1) : a.klen;
     const int rows = a.S * a.kvg, hd = a.l_hd;
-    const double per_group = hd == 128 ? (a.kv_fmt == KV_I8 ? 70e-6 : 117e-6) : hd == 256 ? 76e-6 : 168e-6;    // us per (group, head, key)
+    const double per_group = hd == 128 ? (a.kv_fmt == KV_I8 ? 90e-6 : 117e-6) : hd == 256 ? 76e-6 : 168e-6;    // us per (group, head, key)
     const double t_groups = 8.0 + per_group * ((rows + (hd == 128 ? 23 : 7)) / (hd == 128 ? 24 : 8)) * keys * a.nkv * a.batch;
     const int nq = hd == 128 ? 2 : 1, dsplit = hd == 512 ? 2 : 1, tiles_q = (rows + 127) / 128;
     const bool both = nq == 2 && tiles_q > 1;
@@ -775,15 +777,16 @@ static bool prefers_row_groups(const AttnArgs &a) {
 
 // More query rows per KV head than the decode / verify kernels serve in one CTA (24), no fused append and no partial
 // export.  fp32 queries of 512-wide heads (two fp16 limbs of a query tile do not fit beside the operand ring) run as row
-// groups of the mma.sync kernel, and so do the formats and widths below that these suit better; int8 / head_dim 128, and
-// prefix ranges that only this kernel expresses, always come here.
+// groups of the mma.sync kernel, and so do calls that these suit better.  int8 / head_dim 128 on keys that do not wrap round
+// the ring, and prefix ranges that only this kernel expresses, always come here (no workspace is asked of these calls).
 static bool prefill_eligible(const AttnArgs &a) {
     if (a.no_tma || a.no_tcgen05 || a.block_table != nullptr) return false;
     if (a.new_k != nullptr || a.partial_out != nullptr || a.out == nullptr || a.peer_world > 1) return false;
     if (!a.d0_set && a.S * a.kvg <= 24) return false;
     if (a.kvg != 1 && a.kvg != 2 && a.kvg != 4 && a.kvg != 8) return false;
     if (a.l_hd == 512 && a.q_type != ET_BF16) return false;
-    if ((a.kv_fmt != KV_I8 || a.l_hd != 128) && !a.tcgen05_always && prefers_row_groups(a)) return false;
+    const bool wraps = (long)(a.win_start % a.cache_cap) + a.klen > a.cache_cap;
+    if ((a.kv_fmt != KV_I8 || a.l_hd != 128 || wraps) && !a.d0_set && !a.tcgen05_always && prefers_row_groups(a)) return false;
     const auto al16 = [](const void *x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
     if (!al16(a.k_cache) || !al16(a.v_cache) || !al16(a.q) || !al16(a.out) || a.cache_hd % (a.kv_fmt == KV_I8 ? 16 : 32) != 0) return false;
     if (a.q_batch_stride % 8 != 0 || a.out_batch_stride % 8 != 0 || a.scale_batch_stride % 4 != 0) return false;

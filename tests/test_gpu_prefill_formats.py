@@ -196,3 +196,13 @@ def test_which_kernel_takes_a_prompt_chunk(hd, nh, nkv, fmt, S, klen, window, ch
     a = ops.make_args(q=4096, k_cache=4096, v_cache=4096, k_scales=4096, v_scales=4096, out=4096, kv_fmt={"i8": ops.KV_I8, "i4": ops.KV_I4, "i4b32": ops.KV_I4B32}[fmt],
                       q_type=ops.BF16, out_type=ops.BF16, S=S, nh=nh, nkv=nkv, kvg=nh // nkv, l_hd=hd, cache_hd=hd, cache_cap=klen, klen=klen, window=window)
     assert ops.attn_kernel_choice(a) == choice
+
+
+@pytest.mark.parametrize("nh,nkv,S,klen,window,choice", [
+    (8, 4, 24, 16384, 0, 0), (32, 16, 24, 4096, 0, 0), (32, 16, 128, 4096, 0, 0), (32, 16, 256, 4096, 0, 2), (32, 16, 1024, 2048, 0, 2),
+    (32, 8, 64, 16384, 0, 0), (32, 16, 64, 1088, 1024, 0), (32, 16, 1024, 2048, 1024, 2)])
+def test_which_kernel_takes_a_prompt_chunk_on_a_wrapped_int8_ring(nh, nkv, S, klen, window, choice):
+    cap = klen + 8
+    a = ops.make_args(q=4096, k_cache=4096, v_cache=4096, k_scales=4096, v_scales=4096, out=4096, kv_fmt=ops.KV_I8, q_type=ops.BF16, out_type=ops.BF16,
+                      S=S, nh=nh, nkv=nkv, kvg=nh // nkv, l_hd=128, cache_hd=128, cache_cap=cap, win_start=cap + cap // 2, klen=klen, window=window)
+    assert ops.attn_kernel_choice(a) == choice
