@@ -747,24 +747,32 @@ static int dispatch_mma(cudaStream_t st, const AttnArgs &a, bool q, long *ws) {
 }
 
 // ------------------------------------------------------------------ query-major prefill (attn_prefill_kernel.cuh)
+// Two query tiles to a CTA at head_dim 128, unless every query tile finds an SM of its own, or a head has only one.  Up to one
+// tile per SM one to a CTA is faster throughout (32q/16kv int8 bf16, positions x keys, one / two to a CTA, us: 160 x 4096
+// 68 / 107, 576 x 2048 39 / 58; fp32 queries 160 x 4096 77 / 129), beyond that two: 640 x 2048 61 / 59, 1280 81 / 69, 2048
+// 87 / 69, with a window of 512 640 36 / 29.  (fp32 queries and block-32 caches lose 2 to 7 % by that up to two tiles per SM.)
+static int query_tiles_per_cta(const AttnArgs &a) {
+    const int pos = 128 / a.kvg, tiles = (a.S + pos - 1) / pos;
+    return a.l_hd == 128 && tiles > 1 && (long)tiles * a.nkv * a.batch > device_info().sm_count ? 2 : 1;
+}
 // Estimated time of a call as row groups of the mma.sync kernel against the query-major kernel, in us.  Row groups cost per
 // (group, KV head, key); the query-major kernel per 64-key step of a CTA, with one CTA per SM and no split of the keys, so
 // few query rows against a long cache leave the chip idle.  Constants from launches back to back on one box, 512 / 2048 /
 // 16384 keys x 13 to 256 rows (row groups / query-major, us): 32q/16kv x 256 int8, bf16 queries, 2048 keys: 13 rows 21 / 58,
 // 48 rows 54 / 57, 64 rows 53 / 57, 96 rows 78 / 58, 256 rows 184 / 57; 512 keys: 13 rows 13 / 21, 256 rows 74 / 22;
 // 32q/4kv x 512 block-32, 2048 keys: 64 rows 114 / 132, 96 rows 169 / 132, 256 rows 393 / 134.  int8 x 128, positions x keys,
-// bf16: 32q/16kv 24 x 4096 21 / 81, 24 x 16384 49 / 294, 64 x 4096 46 / 82, 128 x 4096 92 / 107, 256 x 4096 141 / 107,
-// 512 x 2048 126 / 59; 8q/4kv 64 x 16384 37 / 293, 512 x 2048 58 / 59, 1024 x 2048 76 / 59.
+// bf16: 32q/16kv 24 x 16384 49 / 294 and 64 x 4096 46 / 82 (with two query tiles to a CTA), 256 x 4096 141 / 68, 512 x 2048
+// 126 / 39, 1024 x 2048 252 / 60; 8q/4kv 1024 x 2048 76 / 38; int4 32q/16kv 160 x 4096 106 / 70, block-32 135 / 87.
 static bool prefers_row_groups(const AttnArgs &a) {
     const bool b32 = a.kv_fmt == KV_I4B32, f32 = a.q_type == ET_F32;
     const double keys = a.window > 0 ? std::min<long>(a.klen, (long)a.window + a.S - 1) : a.klen;
     const int rows = a.S * a.kvg, hd = a.l_hd;
     const double per_group = hd == 128 ? (a.kv_fmt == KV_I8 ? 90e-6 : 117e-6) : hd == 256 ? 76e-6 : 168e-6;    // us per (group, head, key)
     const double t_groups = 8.0 + per_group * ((rows + (hd == 128 ? 23 : 7)) / (hd == 128 ? 24 : 8)) * keys * a.nkv * a.batch;
-    const int nq = hd == 128 ? 2 : 1, dsplit = hd == 512 ? 2 : 1, tiles_q = (rows + 127) / 128;
-    const bool both = nq == 2 && tiles_q > 1;
+    const int nq = query_tiles_per_cta(a), dsplit = hd == 512 ? 2 : 1, tiles_q = (rows + 127) / 128;
+    const bool both = nq == 2;                         // (a step of two query tiles)
     double step;                                       // us per 64 keys
-    if (hd == 128) step = b32 ? (f32 ? (both ? 3.1 : 2.4) : (both ? 2.1 : 1.4)) : (f32 ? (both ? 1.8 : 1.1) : (both ? 1.45 : 1.05));
+    if (hd == 128) step = b32 ? (f32 ? (both ? 3.1 : 1.4) : (both ? 2.1 : 1.2)) : (f32 ? (both ? 1.8 : 1.15) : (both ? 1.45 : 1.05));
     else if (hd == 256) step = b32 ? (f32 ? 3.0 : 2.2) : (f32 ? 2.0 : 1.5);
     else step = b32 ? 3.8 : 2.1;
     const double ctas = (double)((tiles_q + nq - 1) / nq) * a.nkv * dsplit * a.batch, span = 128.0 * nq / a.kvg;
@@ -809,7 +817,7 @@ static bool prefers_mma(const AttnArgs &a) {
 }
 
 static int dispatch(cudaStream_t st, const AttnArgs &a, bool q, long *ws) {
-    if (!q && prefill_eligible(a)) return launch_attn_prefill(st, a, fault_word());
+    if (!q && prefill_eligible(a)) return launch_attn_prefill(st, a, query_tiles_per_cta(a), fault_word());
     if (a.d0_set) { set_error("this key range needs the prefill kernel (int8 KV, head_dim 128, 16-byte aligned buffers)"); return NOMOS_EUNSUPPORTED; }
     if (!tc5_eligible(a)) return dispatch_mma(st, a, q, ws);
     if (q) {

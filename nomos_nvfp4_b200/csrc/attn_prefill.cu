@@ -10,15 +10,15 @@ using fused::LOG2E;
 
 namespace {
 
-template <int HD, int FMT, int QL>
+template <int HD, int FMT, int QL, int NQ>
 static int launch_prefill_inst(cudaStream_t st, const AttnArgs &a, unsigned int *fault) {
-    using C = pf::Cfg<HD, FMT, QL>;
+    using C = pf::Cfg<HD, FMT, QL, NQ>;
     static bool attr_set[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_set[dev]) {
-        cudaFuncSetAttribute(pf::attn_prefill_kernel<HD, FMT, QL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        cudaFuncSetAttribute(pf::attn_prefill_kernel<HD, FMT, QL, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         attr_set[dev] = true;
     }
     pf::PParams p;
@@ -54,28 +54,30 @@ static int launch_prefill_inst(cudaStream_t st, const AttnArgs &a, unsigned int 
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = st;
     cfg.attrs = pdl; cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, pf::attn_prefill_kernel<HD, FMT, QL>, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, pf::attn_prefill_kernel<HD, FMT, QL, NQ>, p);
     if (e != cudaSuccess) { set_error("attn_prefill launch: %s", cudaGetErrorString(e)); return NOMOS_ECUDA; }
     return NOMOS_OK;
 }
 
 template <int FMT>
-static int launch_prefill_fmt(cudaStream_t st, const AttnArgs &a, unsigned int *fault) {
+static int launch_prefill_fmt(cudaStream_t st, const AttnArgs &a, int query_tiles, unsigned int *fault) {
     const bool one = a.q_type == ET_BF16;              // bf16 query rows fit one fp16 limb exactly
     switch (a.l_hd) {
-        case 128: return one ? launch_prefill_inst<128, FMT, 1>(st, a, fault) : launch_prefill_inst<128, FMT, 2>(st, a, fault);
-        case 256: return one ? launch_prefill_inst<256, FMT, 1>(st, a, fault) : launch_prefill_inst<256, FMT, 2>(st, a, fault);
-        default: return launch_prefill_inst<512, FMT, 1>(st, a, fault);
+        case 128:
+            if (query_tiles == 1) return one ? launch_prefill_inst<128, FMT, 1, 1>(st, a, fault) : launch_prefill_inst<128, FMT, 2, 1>(st, a, fault);
+            return one ? launch_prefill_inst<128, FMT, 1, 2>(st, a, fault) : launch_prefill_inst<128, FMT, 2, 2>(st, a, fault);
+        case 256: return one ? launch_prefill_inst<256, FMT, 1, 1>(st, a, fault) : launch_prefill_inst<256, FMT, 2, 1>(st, a, fault);
+        default: return launch_prefill_inst<512, FMT, 1, 1>(st, a, fault);
     }
 }
 
 }  // namespace
 
-int launch_attn_prefill(cudaStream_t st, const AttnArgs &a, unsigned int *fault) {
+int launch_attn_prefill(cudaStream_t st, const AttnArgs &a, int query_tiles, unsigned int *fault) {
     switch (a.kv_fmt) {
-        case KV_I8: return launch_prefill_fmt<KV_I8>(st, a, fault);
-        case KV_I4: return launch_prefill_fmt<KV_I4>(st, a, fault);
-        default: return launch_prefill_fmt<KV_I4B32>(st, a, fault);
+        case KV_I8: return launch_prefill_fmt<KV_I8>(st, a, query_tiles, fault);
+        case KV_I4: return launch_prefill_fmt<KV_I4>(st, a, query_tiles, fault);
+        default: return launch_prefill_fmt<KV_I4B32>(st, a, query_tiles, fault);
     }
 }
 

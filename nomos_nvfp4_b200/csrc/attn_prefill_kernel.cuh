@@ -49,11 +49,14 @@ constexpr int SMEM_MAX = 232448;              // shared memory a CTA may ask for
 
 constexpr int cmin(int a, int b) { return a < b ? a : b; }
 
-template <int HD_, int FMT_, int QL_>
+template <int HD_, int FMT_, int QL_, int NQ_>
 struct Cfg {
     static constexpr int HD = HD_, FMT = FMT_, QL = QL_;               // QL: fp16 limbs of the query
     static constexpr int KL = FMT == KV_I4B32 ? 2 : 1;                 // fp16 limbs of K and V
-    static constexpr int NQ = HD == 128 ? 2 : 1;                       // query tiles per CTA
+    // Query tiles per CTA.  Two share a CTA's K and V slots at head_dim 128 (64 keys x 256 rows 1.45 us, 128 rows 1.05 us), but
+    // where all query tiles find an SM of their own the CTA with one is done sooner.
+    static constexpr int NQ = NQ_;
+    static_assert(NQ == 1 || (NQ == 2 && HD == 128), "tensor memory columns");
     static constexpr int DV = cmin(HD, 256);                           // output dims per CTA
     static constexpr int DSPLIT = HD / DV;
     static constexpr int Q_BLOCK = MR * 128;                           // 64 dims of a query tile (one swizzle block column)
@@ -301,10 +304,10 @@ __device__ __noinline__ void add_nonfinite_values(const PParams &p) {
     }
 }
 
-template <int HD, int FMT, int QL>
-__global__ void __launch_bounds__(Cfg<HD, FMT, QL>::NTHREADS, 1) attn_prefill_kernel(const __grid_constant__ PParams p) {
-    using C = Cfg<HD, FMT, QL>;
-    constexpr int NQ = C::NQ, NSB = C::NSB, NSLOT = C::NSLOT, KL = C::KL, DV = C::DV, NCONST = C::NCONST;
+template <int HD, int FMT, int QL, int NQ>
+__global__ void __launch_bounds__(Cfg<HD, FMT, QL, NQ>::NTHREADS, 1) attn_prefill_kernel(const __grid_constant__ PParams p) {
+    using C = Cfg<HD, FMT, QL, NQ>;
+    constexpr int NSB = C::NSB, NSLOT = C::NSLOT, KL = C::KL, DV = C::DV, NCONST = C::NCONST;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = smem_raw;
     const uint32_t sm_u32 = smem_u32(sm);

@@ -90,8 +90,9 @@ struct LaunchInfo { int kernel, splits, merge_route; };
 LaunchInfo attn_last_launch_info();
 int attn_kernel_choice(const AttnArgs &a);     // 2: the query-major prefill kernel, 1: the tcgen05 decode / verify kernel, 0: the mma.sync kernel
 int launch_attn_fused(cudaStream_t st, const AttnArgs &a);
-// attn_prefill.cu: the query-major prefill kernel, for calls attn_fused.cu found eligible; `fault` is the device fault word
-int launch_attn_prefill(cudaStream_t st, const AttnArgs &a, unsigned int *fault);
+// attn_prefill.cu: the query-major prefill kernel, for calls attn_fused.cu found eligible, with `query_tiles` (1; 2 at head_dim
+// 128 only) tiles of 128 rows per CTA; `fault` is the device fault word
+int launch_attn_prefill(cudaStream_t st, const AttnArgs &a, int query_tiles, unsigned int *fault);
 long attn_paged_workspace_bytes(const AttnArgs &a);
 int launch_attn_paged(cudaStream_t st, const AttnArgs &a);
 // Reads (and optionally clears) the device word the kernels OR into when a bounded wait runs out.

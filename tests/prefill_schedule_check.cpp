@@ -82,7 +82,7 @@ int main() {
     int walks = 0;
     for (int n = 1; n <= 23; ++n) {
         const TileRange all[1] = {{0, n - 1}};
-        walks += walk<1, 2, 2>(n, all) + walk<1, 4, 2>(n, all);
+        walks += walk<1, 1, 1>(n, all) + walk<1, 2, 2>(n, all) + walk<1, 4, 2>(n, all);
         // two query tiles: either may start later or end earlier, or have no keys at all
         for (int a = 0; a <= n; ++a)
             for (int b = 0; b <= n; ++b) {

@@ -54,6 +54,21 @@ def test_formats_and_head_dims(oracle, fmt, hd, q_type, S, klen, window, kvg):
     check(oracle, c, q, got[0], S=S, klen=klen, start=0, window=window, scale=scale, bf16_out=q_type == ops.BF16)
 
 
+@pytest.mark.parametrize("q_type", [ops.F32, ops.BF16])
+@pytest.mark.parametrize("fmt", ["i8", "i4", "i4b32"])
+@pytest.mark.parametrize("S,klen,window,kvg,nkv", [(576, 576, 0, 2, 16), (640, 640, 0, 2, 16), (129, 200, 0, 8, 20), (290, 430, 60, 4, 16)])
+def test_one_and_two_query_tiles_per_cta(oracle, fmt, q_type, S, klen, window, kvg, nkv):
+    """head_dim 128 on both sides of the size where CTAs take two query tiles (more tiles than the chip's 148 SMs: 144 in the
+    first case, then 160, 180 with every head's last CTA half empty, 160); keys wrapped round the ring."""
+    rng = np.random.default_rng(S + kvg)
+    c = build_cache(fmt, rng, klen, nkv, 128, cap=klen + 5, start=klen + 9)
+    q = bf16_normal(rng, (S, nkv * kvg, 128))
+    scale = 1.0 / np.sqrt(128)
+    got, choice = run_fused(c, q, S=S, klen=klen, win_start=klen + 9, window=window, scale=scale, q_type=q_type, out_type=q_type, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    check(oracle, c, q, got[0], S=S, klen=klen, start=klen + 9, window=window, scale=scale, bf16_out=q_type == ops.BF16)
+
+
 @pytest.mark.parametrize("hd,fmt,q_type", [(128, "i8", ops.F32), (128, "i4b32", ops.BF16), (256, "i4b32", ops.F32), (512, "i4", ops.BF16)])
 def test_wrapped_ring(oracle, hd, fmt, q_type):
     """The window's keys run past the end of the ring: rows are addressed one by one."""
