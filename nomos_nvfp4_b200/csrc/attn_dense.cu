@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(DW * 32) attn_dense_kernel(const DParams p) {
 #pragma unroll
             for (int w = 0; w < NST; ++w) o += wgt[w] * so[w][j][d];
             if (p.splits > 1) p.part_o[((size_t)split * p.grows + grow) * HD + d] = o;
-            else p.out[grow * HD + d] = lstar > 0.0f ? o / lstar : 0.0f;
+            else p.out[grow * HD + d] = lstar == 0.0f ? 0.0f : o / lstar;      // (a NaN stays one)
         }
         if (p.splits > 1 && threadIdx.x == 0) {
             p.part_ml[((size_t)split * p.grows + grow) * 2] = mstar;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) dense_merge_kernel(const DParams p) {
     float l = 0.0f;
     for (int i = tid; i < p.splits; i += 256) {
         const float2 ml = *reinterpret_cast<const float2 *>(p.part_ml + ((size_t)i * p.grows + row) * 2);
-        const float w = ml.y > 0.0f ? ex2f(ml.x - m) : 0.0f;
+        const float w = ml.y == 0.0f ? 0.0f : ex2f(ml.x - m);          // (no key in the split; a NaN stays one)
         wgt[i] = w;
         l = fmaf(w, ml.y, l);
     }
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) dense_merge_kernel(const DParams p) {
         float o = 0.0f;
 #pragma unroll
         for (int k = 0; k < NG; ++k) o += reinterpret_cast<const float *>(part[k])[d];
-        p.out[(size_t)row * HD + d] = l > 0.0f ? o / l : 0.0f;
+        p.out[(size_t)row * HD + d] = l == 0.0f ? 0.0f : o / l;
     }
 }
 

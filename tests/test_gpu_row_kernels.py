@@ -56,6 +56,31 @@ def test_dense_decode_key_counts(dtype, nh, nkv, hd, T):
     assert (out.double() - want).abs().max().item() <= 1e-5 * want.square().mean().sqrt().item()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("S,T", [(1, 40), (1, 4099), (37, 400)])
+def test_dense_a_nan_stays_one(dtype, S, T):
+    """A NaN or infinite key: rows that see it are NaN whatever the number of splits, heads and rows that do not are bit for
+    bit what they are without it."""
+    g = torch.Generator(device=DEV); g.manual_seed(S + T)
+    nh, nkv, hd, key = 4, 2, 128, T - (S + 1) // 2
+    k, v = (torch.randn(nkv, T, hd, generator=g, device=DEV).to(dtype) for _ in range(2))
+    q = torch.randn(S, nh, hd, generator=g, device=DEV) * hd ** -0.5
+    scratch = torch.empty(S * nh * T, device=DEV)
+    f = ops.attention_prefill_prefix_batched_fp32 if dtype == torch.float32 else ops.attention_prefill_prefix_batched_bf16
+    outs = []
+    for bad in (None, float("nan"), float("inf")):
+        if bad is not None:
+            k[0, key] = bad
+        out = torch.full((S, nh, hd), -1e30, device=DEV)
+        a = (q, 0, scratch, 0, out, k, v) if dtype == torch.float32 else (q, 0, 0, scratch, 0, 0, out, k, v)
+        f(None, None, *a, nh, nkv, hd, hd, T, S, T, nh // nkv, 0, T - S, 0)
+        outs.append(host(out))
+    sees = np.zeros((S, nh), bool)
+    sees[np.arange(S) + T - S >= key, :nh // nkv] = True
+    for got in outs[1:]:
+        assert np.array_equal(got[~sees], outs[0][~sees]) and np.isnan(got[sees]).all() and sees.any()
+
+
 @pytest.mark.parametrize("hd,shift", [(128, 0), (512, 0), (256, 8)])
 def test_block32_reader_to_int8_every_code(oracle, hd, shift):
     """All 16 nibble values under scales from subnormal to large, aligned rows (table kernel) and rows 8 bytes off (general
