@@ -6,7 +6,9 @@ These tests put real producers in front of it and check every step of the chain 
   * the producer epilogue rewrites the query IN PLACE and appends the newest rows, then the tcgen05 kernel
     (and the mma.sync kernel) reads them -- one query buffer reused by every step;
   * a decode loop on ONE cache where every step's attention call carries its own fused append and sets
-    NOMOS_ATTN_SETTLED_CACHE, so step i+1 must not stream the row step i is still storing.
+    NOMOS_ATTN_SETTLED_CACHE, so step i+1 must not stream the row step i is still storing;
+  * the same loop with the append as a call of its own (it lets the attention grid start early and writes other rows
+    to other slots in every step), linear caches, wrapped rings and paged caches.
 """
 import numpy as np
 import pytest
@@ -119,3 +121,93 @@ def test_single_cache_fused_append_loop_with_settled_cache_flag(oracle, path, n_
             ok, rel = within(got[i][r], want[r], TOL)
             assert ok, f"step {i} row {r}: {rel:.2e} x RMS"
     assert np.array_equal(host(ck).view(np.uint8), c.k.view(np.uint8)) and np.array_equal(host(cks), c.ks)
+
+
+@pytest.mark.parametrize("fmt,hd,nh,nkv,path", [("i8", 128, 8, 4, "mma_sync"), ("i8", 128, 8, 4, "tcgen05"), ("i4", 256, 4, 2, "auto"), ("i4b32", 256, 8, 4, "auto"),
+                                               ("i4b32", 512, 8, 2, "auto")])
+@pytest.mark.parametrize("n_s,window", [(1, 0), (9, 0), (1, 300), (9, 300)])
+def test_append_call_then_attention_loop_with_settled_cache_flag(oracle, fmt, hd, nh, nkv, path, n_s, window):
+    """append, attention, append, attention, ... without synchronisation: the append releases the attention grid before it
+    has written a byte, and step i + 1's append must not overwrite a ring slot that step i still reads."""
+    rng = np.random.default_rng(180 + n_s + hd + window)
+    steps, T0 = 10, 1149
+    cap = window + n_s - 1 if window else T0 + steps * n_s
+    c = KVCache(fmt, nkv, cap, hd)
+    first = max(0, T0 - cap) if window else 0
+    c.append(bf16_normal(rng, (T0 - first, nkv, hd)), bf16_normal(rng, (T0 - first, nkv, hd)), first)
+    ck, cv, cks, cvs = dev(c.k), dev(c.v), dev(c.ks), dev(c.vs)
+    q = bf16_normal(rng, (steps, n_s, nh, hd))
+    nk, nv = bf16_normal(rng, (steps, n_s, nkv, hd)), bf16_normal(rng, (steps, n_s, nkv, hd))
+    dq, dnk, dnv = dev(q), dev(nk), dev(nv)
+    outs = torch.full((steps, n_s, nh, hd), -1e30, dtype=torch.float32, device=DEV)
+    args = []
+    for i in range(steps):
+        end = T0 + (i + 1) * n_s
+        klen = min(cap, end)
+        args.append(ops.make_args(q=dq[i], k_cache=ck, v_cache=cv, k_scales=cks, v_scales=cvs, out=outs[i], kv_fmt=c.kv_fmt, S=n_s, nh=nh, nkv=nkv, kvg=nh // nkv,
+                                  l_hd=hd, cache_hd=hd, cache_cap=cap, win_start=end - klen, klen=klen, window=window, softmax_scale=0.1,
+                                  flags=PATHS[path] | ops.SETTLED_CACHE))
+    need = max(ops.attn_workspace_bytes(a) for a in args)
+    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=DEV)
+    for a in args:
+        a.workspace, a.ws_bytes = ws.data_ptr(), need
+    torch.cuda.synchronize()
+    for i, a in enumerate(args):
+        rows = (dnk[i], dnv[i], ck, cv, cks, cvs, n_s, nkv, hd, nkv * hd, cap, hd, T0 + i * n_s)
+        if fmt == "i8":
+            ops.gpu_append_quant_kv_i8(None, *rows)
+        else:
+            ops.gpu_append_quant_kv_i4(None, *rows, c.scale_blocks)
+        ops.attn_fused(None, a)
+    torch.cuda.synchronize()
+    got = host(outs)
+    for i in range(steps):
+        c.append(nk[i], nv[i], T0 + i * n_s)
+        end = T0 + (i + 1) * n_s
+        want = oracle.attn_exact(q[i], c.k, c.v, c.ks, c.vs, c.kv_fmt, nh, nkv, hd, hd, cap, S=n_s, window=window, query_base_pos=end - n_s,
+                                 win_lo=end - min(cap, end), softmax_scale=0.1)
+        for r in range(n_s):
+            ok, rel = within(got[i][r], want[r], TOL)
+            assert ok, f"step {i} row {r}: {rel:.2e} x RMS"
+    for d, h in ((ck, c.k), (cv, c.v), (cks, c.ks), (cvs, c.vs)):
+        assert np.array_equal(host(d).view(np.uint8), h.view(np.uint8))
+
+
+def test_paged_append_then_paged_attention_loop(oracle):
+    rng = np.random.default_rng(190)
+    nkv, hd, nh, steps, lens0 = 4, 128, 8, 10, [125, 300, 1200]
+    page, per, batch = 128, 11, 3
+    table = rng.permutation(batch * per).astype(np.int32).reshape(batch, per)
+    caches = [KVCache("i8", nkv, per * page, hd) for _ in range(batch)]
+    pools = np.zeros((2, batch * per, nkv, page, hd), np.int8)
+    spools = np.ones((2, batch * per, nkv, page), np.float32)
+    for b, (c, n) in enumerate(zip(caches, lens0)):
+        c.append(bf16_normal(rng, (n, nkv, hd)), bf16_normal(rng, (n, nkv, hd)), 0)
+        for j in range(per):
+            at = slice(j * page, (j + 1) * page)
+            pools[0, table[b, j]], pools[1, table[b, j]] = c.k[:, at], c.v[:, at]
+            spools[0, table[b, j]], spools[1, table[b, j]] = c.row_scales_f32("k")[:, at], c.row_scales_f32("v")[:, at]
+    q = bf16_normal(rng, (steps, batch, nh, hd))
+    nk, nv = bf16_normal(rng, (steps, batch, nkv, hd)), bf16_normal(rng, (steps, batch, nkv, hd))
+    dq, dnk, dnv, dt = dev(q), dev(nk), dev(nv), dev(table)
+    kp, vp, ksp, vsp = dev(pools[0]), dev(pools[1]), dev(spools[0]), dev(spools[1])
+    pos = dev(np.array([[n + i for n in lens0] for i in range(steps)], np.int32))
+    lens = pos + 1
+    outs = torch.full((steps, batch, nh, hd), -1e30, dtype=torch.float32, device=DEV)
+    max_len = max(lens0) + steps
+    wsb = ops.attn_paged_workspace_bytes(batch, nh, nkv, nh // nkv, hd, max_len)
+    ws = torch.empty(max(wsb, 16), dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    for i in range(steps):
+        ops.kv_paged_append_quant_i8(None, dnk[i], dnv[i], kp, vp, ksp, vsp, dt, pos[i], batch=batch, nkv=nkv, l_hd=hd, l_kvd=nkv * hd, max_pages=per)
+        ops.attn_paged_decode_i8(None, dq[i], kp, vp, ksp, vsp, dt, lens[i], outs[i], ws, wsb, batch=batch, nh=nh, nkv=nkv, kvg=nh // nkv, l_hd=hd,
+                                 n_pages=batch * per, max_pages=per, max_len=max_len, softmax_scale=0.1)
+    torch.cuda.synchronize()
+    got = host(outs)
+    for i in range(steps):
+        for b, c in enumerate(caches):
+            n = lens0[b] + i
+            c.append(nk[i, b][None], nv[i, b][None], n)
+            want = oracle.attn_exact(q[i, b][None], c.k, c.v, c.ks, c.vs, c.kv_fmt, nh, nkv, hd, hd, per * page, S=1, query_base_pos=n, softmax_scale=0.1)
+            ok, rel = within(got[i, b][None], want, TOL)
+            assert ok, f"step {i} sequence {b}: {rel:.2e} x RMS"

@@ -1,5 +1,5 @@
 """The query-major prefill kernel over every cache format and head dim it serves, at the edges of its tiles: query tiles
-of 128 rows (two per CTA at head_dim 128), key tiles of 64 or 128 keys, ragged ends, windows, wrapped rings, one and two
+of 128 rows (one or two per CTA at head_dim 128), key tiles of 64 keys, ragged ends, windows, wrapped rings, one and two
 query limbs.  Checked against the oracle's fp64 attention over the same cache bytes.
 
 Tolerance: 2e-4 x RMS per row for fp32 outputs.  The operands carry the codes, the block scales and bf16 queries exactly,
@@ -11,7 +11,7 @@ import torch
 
 from nomos_nvfp4_b200 import ops
 from tests._cases import KVCache, bf16_normal
-from tests._gpu import within
+from tests._gpu import DEV, dev, host, within
 from tests.test_gpu_attn import build_cache
 from tests.test_gpu_prefill import SENTINEL, run_fused
 
@@ -80,6 +80,58 @@ def test_wrapped_ring(oracle, hd, fmt, q_type):
     got, choice = run_fused(c, q, S=S, klen=klen, win_start=start, window=window, scale=scale, q_type=q_type, out_type=q_type, flags=ops.TCGEN05_ALWAYS)
     assert choice == 2
     check(oracle, c, q, got[0], S=S, klen=klen, start=start, window=window, scale=scale, bf16_out=q_type == ops.BF16)
+
+
+@pytest.mark.parametrize("hd,fmt,q_type", [(128, "i8", ops.BF16), (128, "i4b32", ops.F32), (256, "i4", ops.BF16), (256, "i4b32", ops.F32), (512, "i4b32", ops.BF16), (512, "i8", ops.BF16)])
+def test_batch_strides_and_a_wide_row_pitch(oracle, hd, fmt, q_type):
+    """Two sequences with padded strides, cache rows wider than the head dim, and values of mean 2 (sums over all tiles)."""
+    rng = np.random.default_rng(hd + 8)
+    nkv, kvg, S, T, batch, cache_hd = 2, 2, 70, 203, 2, hd + 64
+    nh, scale = nkv * kvg, 1.0 / np.sqrt(hd)
+    cs = []
+    for _ in range(batch):
+        c = KVCache(fmt, nkv, T + 5, hd, cache_hd)
+        c.append(bf16_normal(rng, (T, nkv, hd)), bf16_normal(rng, (T, nkv, hd)) + np.float32(2), 0)
+        cs.append(c)
+    q = bf16_normal(rng, (batch, S, nh, hd))
+
+    def padded(arrays, pad):
+        n = arrays[0].size * arrays[0].itemsize
+        buf = np.full((len(arrays), n + pad), 0x55, np.uint8)
+        for i, a in enumerate(arrays):
+            buf[i, :n] = np.frombuffer(np.ascontiguousarray(a).tobytes(), np.uint8)
+        return dev(buf), n + pad
+    (k, kstride), (v, _) = padded([c.k for c in cs], 96), padded([c.v for c in cs], 96)
+    (ks, sstride), (vs, _) = padded([c.ks for c in cs], 20), padded([c.vs for c in cs], 20)
+    qs, os_ = S * nh * hd + 24, S * nh * hd + 40
+    tt = torch.bfloat16 if q_type == ops.BF16 else torch.float32
+    dq = torch.full((batch, qs), 7.0, dtype=tt, device=DEV)
+    dq[:, :S * nh * hd] = dev(q.reshape(batch, -1)).to(tt)
+    out = torch.full((batch, os_), SENTINEL, dtype=torch.float32, device=DEV)
+    a = ops.make_args(q=dq, k_cache=k, v_cache=v, k_scales=ks, v_scales=vs, out=out, kv_fmt=cs[0].kv_fmt, q_type=q_type, out_type=ops.F32, batch=batch, S=S, nh=nh,
+                      nkv=nkv, kvg=kvg, l_hd=hd, cache_hd=cache_hd, cache_cap=T + 5, klen=T, softmax_scale=scale, q_batch_stride=qs, out_batch_stride=os_,
+                      kv_batch_stride=kstride, scale_batch_stride=sstride, flags=ops.TCGEN05_ALWAYS)
+    assert ops.attn_kernel_choice(a) == 2
+    ops.attn_fused(None, a)
+    torch.cuda.synchronize()
+    got = host(out)
+    assert np.all(got[:, S * nh * hd:] == SENTINEL)
+    for b, c in enumerate(cs):
+        check(oracle, c, q[b], got[b, :S * nh * hd].reshape(S, nh, hd), S=S, klen=T, start=0, window=0, scale=scale, bf16_out=False)
+
+
+@pytest.mark.parametrize("hd,fmt", [(256, "i8"), (256, "i4b32"), (512, "i4b32"), (512, "i4")])
+def test_long_caches_and_values_of_one_sign(oracle, hd, fmt):
+    """6000 keys in front of the chunk, values of mean 2: the fp32 sums of O run over a hundred tiles in tensor memory and no
+    longer cancel.  T terms of one sign in fp32: T / 64 roundings of 2^-24 at the value's size, 6e-6 of it, within TOL."""
+    rng = np.random.default_rng(hd + 9)
+    nkv, kvg, S, T = 1, 4, 40, 6011
+    c = KVCache(fmt, nkv, T, hd)
+    c.append(bf16_normal(rng, (T, nkv, hd)), bf16_normal(rng, (T, nkv, hd)) + np.float32(2), 0)
+    q, scale = bf16_normal(rng, (S, nkv * kvg, hd)), 1.0 / np.sqrt(hd)
+    got, choice = run_fused(c, q, S=S, klen=T, scale=scale, q_type=ops.BF16, flags=ops.TCGEN05_ALWAYS)
+    assert choice == 2
+    check(oracle, c, q, got[0], S=S, klen=T, start=0, window=0, scale=scale, bf16_out=False)
 
 
 @pytest.mark.parametrize("hd,fmt", [(128, "i8"), (256, "i4"), (512, "i4b32")])

@@ -81,15 +81,19 @@ def test_dense_a_nan_stays_one(dtype, S, T):
         assert np.array_equal(got[~sees], outs[0][~sees]) and np.isnan(got[sees]).all() and sees.any()
 
 
+@pytest.mark.parametrize("special", [False, True])
 @pytest.mark.parametrize("hd,shift", [(128, 0), (512, 0), (256, 8)])
-def test_block32_reader_to_int8_every_code(oracle, hd, shift):
-    """All 16 nibble values under scales from subnormal to large, aligned rows (table kernel) and rows 8 bytes off (general
+def test_block32_reader_to_int8_every_code(oracle, hd, shift, special):
+    """All 16 nibble values under scales from subnormal to large (special: also infinite and zero), aligned rows (table kernel) and rows 8 bytes off (general
     kernel): the same bytes from both, and the reference's arithmetic (multiply, divide, round away) in float32."""
     rng = np.random.default_rng(hd)
     nkv, cap, klen, start, nb = 2, 37, 29, 20, hd // 32
     codes = rng.integers(0, 256, (nkv, cap, hd // 2), dtype=np.uint8)
     s16 = (2.0 ** rng.uniform(-16, 6, (nkv, cap, nb))).astype(np.float16)
+    if special:                                        # overflowed and empty blocks, rows of zeros
+        s16[0, ::5, 0], s16[0, 1::5, 1], s16[1, ::7] = np.inf, 0, 0
     q8 = (s16.astype(np.float32).max(-1) * np.float32(7.0) / np.float32(127.0)).astype(np.float32)
+    q8[q8 == 0] = 1
     scales = np.concatenate([s16.view(np.uint8).ravel(), q8.view(np.uint8).ravel()])
     raw = torch.zeros(codes.size + 64, dtype=torch.uint8, device=DEV)
     raw[shift:shift + codes.size] = dev(codes.ravel())
@@ -99,6 +103,8 @@ def test_block32_reader_to_int8_every_code(oracle, hd, shift):
     slots = (start + np.arange(klen)) % cap
     nib = np.stack([codes & 15, codes >> 4], -1).reshape(nkv, cap, hd).astype(np.int32)
     q = ((nib ^ 8) - 8).astype(np.float32)
-    x = (q * np.repeat(s16.astype(np.float32), 32, -1)) / q8[..., None]
-    want = np.clip(np.trunc(x + np.where(x >= 0, np.float32(0.5), np.float32(-0.5)).astype(np.float32)), -127, 127).astype(np.int8)
+    with np.errstate(invalid="ignore"):
+        x = (q * np.repeat(s16.astype(np.float32), 32, -1)) / q8[..., None]
+        y = np.trunc(x + np.where(x >= 0, np.float32(0.5), np.float32(-0.5)).astype(np.float32))
+    want = np.clip(np.where(np.isnan(y), 0, y), -127, 127).astype(np.int8)      # (a NaN converts to 0)
     assert np.array_equal(host(out), want[:, slots]) and np.array_equal(host(osc), q8[:, slots])
