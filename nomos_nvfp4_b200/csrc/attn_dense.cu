@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(DW * 32) attn_dense_kernel(const DParams p) {
     }
 }
 
-// Merge of the splits: one CTA per query row, eight groups of threads over the splits.
+// Merge of the splits: one CTA per query row, NG groups of threads over the splits.
 constexpr int MERGE_MAX = 512;        // most splits
 template <int HD>
 __global__ void __launch_bounds__(256) dense_merge_kernel(const DParams p) {

@@ -1,6 +1,6 @@
 // Query-major flash prefill straight off the packed KV cache on the fifth-generation tensor cores (tcgen05 + tensor
-// memory), sm_100a: int8, int4 and block-32 int4 caches, head dims 128 / 256 / 512.  The host side (eligibility, launch)
-// is in attn_fused.cu.
+// memory), sm_100a: int8, int4 and block-32 int4 caches, head dims 128 / 256 / 512.  Which calls come here
+// is decided in attn_fused.cu, the launch is in attn_prefill.cu.
 //
 // Replaces the reference's square / prefix batched prefill attention
 //   lib/attention_gpu_int8.mojo:804-887 (int8), lib/batched_attn_gpu.mojo:448-666 (fp32 / bf16 twins)
@@ -20,13 +20,14 @@
 // The value scale rides in the exponent: with u' = logit + log2(vscale) the weight is w = 2^(u' - m), m a whole-number
 // running reference of u', so w fits fp16 whatever the scale, and the denominator takes w / vscale.
 //
-// Roles: per query tile four softmax warps (thread = query row = TMEM lane: S is read 32 columns at a time and the
-// weights go back into the SAME columns, hi and lo, as the A operand of PV); "dequant" warps that fetch cache bytes
-// from global memory one operand slot ahead, widen them and fill a ring of K / V slots in the order the tensor core
-// takes them (rows are addressed one by one: rings may wrap); one MMA warp.  head_dim 128: two query tiles per CTA in
-// turn, one tile's softmax under the other's products; wider heads: one query tile with four S buffers, and at 512 two
-// CTAs per query tile that each own 256 output dims.  The order of products and waits is prefill_schedule.h.  O stays in tensor memory; it is rescaled in place only when a
-// row's reference moves, which happens when a chunk exceeds it by more than 2^8 (a handful of times per row).
+// Roles: per query tile eight softmax warps of 16 rows (a thread holds two rows and every fourth pair of keys; the weights
+// go back into the SAME columns as S, hi and lo, as the A operand of PV); "dequant" warps in teams of two that fetch cache
+// bytes from global memory ahead of their turn, widen them and fill a ring of K / V slots in the order the tensor core
+// takes them (rows are addressed one by one: rings may wrap); one MMA warp.  head_dim 128: one query tile per CTA, or two
+// in turn, one tile's softmax under the other's products; at 512 two CTAs per query tile that each own 256 output dims.
+// Four S buffers, shared by the query tiles; the order of products and waits is prefill_schedule.h.  O stays in tensor
+// memory; it is rescaled in place only when a row's reference moves, which happens when a chunk exceeds it by more than
+// 2^8 (a handful of times per row).
 // Every wait is an mbarrier wait with a time limit; a wait that runs out raises the CTA's abort flag and bit 1 of the
 // device fault word, every role leaves its loop, tensor memory is freed and the CTA exits.
 #pragma once
@@ -150,12 +151,6 @@ __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(pred));
     return pred != 0;
-}
-// This warp's 32 TMEM lanes x 32 consecutive 32-bit columns: thread t gets lane t's row.  The caller waits.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
 }
 // 16 lanes x 8 n columns, spread over the warp like an MMA accumulator: registers 4 e + 2 r + {0, 1} of a thread are
 // columns 8 e + 2 (lane % 4) + {0, 1} of row 8 r + lane / 4.  The caller waits.
@@ -398,37 +393,33 @@ __global__ void __launch_bounds__(Cfg<HD, FMT, QL, NQ>::NTHREADS, 1) attn_prefil
         // S buffer buf += dims 128 c .. 128 c + 127 of query tile g x the K slots from n on
         auto qk = [&](int g, int buf, int c, int n) {
             const uint32_t d = tmem_base + C::TMEM_S + buf * KT;
-            {
 #pragma unroll
-                for (int kl = 0; kl < KL; ++kl) {
-                    const uint64_t bd = rdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
+            for (int kl = 0; kl < KL; ++kl) {
+                const uint64_t bd = rdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
 #pragma unroll
-                    for (int ql = 0; ql < QL; ++ql) {
-                        if (ql + kl > 1) continue;                     // low x low: 2^-18 of the logit's terms and less
-                        const uint64_t ad = qdesc + (uint64_t)(((g * QL + ql) * C::Q_LIMB + 2 * c * C::Q_BLOCK) >> 4);
+                for (int ql = 0; ql < QL; ++ql) {
+                    if (ql + kl > 1) continue;                         // low x low: 2^-18 of the logit's terms and less
+                    const uint64_t ad = qdesc + (uint64_t)(((g * QL + ql) * C::Q_LIMB + 2 * c * C::Q_BLOCK) >> 4);
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            umma_f16(d, ad + (uint64_t)(((k >> 2) * C::Q_BLOCK >> 4) + (k & 3) * 2), bd + (uint64_t)(((k >> 2) * C::BLOCK >> 4) + (k & 3) * 2),
-                                     idesc_qk, (c | kl | ql | k) != 0 ? 1u : 0u);
-                    }
+                    for (int k = 0; k < 8; ++k)
+                        umma_f16(d, ad + (uint64_t)(((k >> 2) * C::Q_BLOCK >> 4) + (k & 3) * 2), bd + (uint64_t)(((k >> 2) * C::BLOCK >> 4) + (k & 3) * 2),
+                                 idesc_qk, (c | kl | ql | k) != 0 ? 1u : 0u);
                 }
             }
         };
         // dims 128 c .. of O of query tile g += P in S buffer buf x the V slots from n on
         auto pv = [&](int g, int buf, int c, int n, bool first) {
             const uint32_t a = tmem_base + C::TMEM_S + buf * KT;
-            {
 #pragma unroll
-                for (int kl = 0; kl < KL; ++kl) {
-                    const uint64_t bd = vrdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
+            for (int kl = 0; kl < KL; ++kl) {
+                const uint64_t bd = vrdesc + (uint64_t)((n + kl) * (C::SLOT >> 4));
 #pragma unroll
-                    for (int pl = 0; pl < 2; ++pl) {
-                        if (pl + kl > 1) continue;
+                for (int pl = 0; pl < 2; ++pl) {
+                    if (pl + kl > 1) continue;
 #pragma unroll
-                        for (int k = 0; k < KT / 16; ++k)              // 16 keys: 8 columns of A, 2048 bytes of the MN-major blocks
-                            umma_f16_ts(tmem_base + C::TMEM_O + g * DV + c * 128, a + 32 * pl + 8 * k, bd + (uint64_t)(k * (2048 >> 4)),
-                                        idesc_pv, (!first || kl || pl || k) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < KT / 16; ++k)                  // 16 keys: 8 columns of A, 2048 bytes of the MN-major blocks
+                        umma_f16_ts(tmem_base + C::TMEM_O + g * DV + c * 128, a + 32 * pl + 8 * k, bd + (uint64_t)(k * (2048 >> 4)),
+                                    idesc_pv, (!first || kl || pl || k) ? 1u : 0u);
                 }
             }
         };

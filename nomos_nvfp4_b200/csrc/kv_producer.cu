@@ -224,6 +224,15 @@ static bool producer_rows_ok(const ProducerArgs &a) {
     return a.cache_hd % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.dst_k) | reinterpret_cast<uintptr_t>(a.dst_v)) & 3) == 0;
 }
 
+static int sm_count() {
+    static int sms[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (sms[dev] == 0 && (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms[dev] <= 0)) sms[dev] = 148;
+    return sms[dev];
+}
+
 int launch_kv_producer(cudaStream_t st, const ProducerArgs &a) {
     cudaLaunchAttribute pdl[1];
     pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -236,7 +245,7 @@ int launch_kv_producer(cudaStream_t st, const ProducerArgs &a) {
     if (producer_rows_ok(a)) {
         // few tokens: a warp per row (latency); many: fewer, longer CTAs per token, down to one, while they still fill the chip
         const int most = (rows + WARPS - 1) / WARPS;
-        const int gx = std::max(1, std::min(most, (4 * 148 + a.n_s - 1) / a.n_s));
+        const int gx = std::max(1, std::min(most, (4 * sm_count() + a.n_s - 1) / a.n_s));
         cfg.gridDim = dim3((unsigned)((long)gx * a.n_s)); cfg.blockDim = dim3(WARPS * 32);
         e = a.l_hd == 128 ? cudaLaunchKernelEx(&cfg, kv_producer_kernel<128>, a, gx)
             : a.l_hd == 256 ? cudaLaunchKernelEx(&cfg, kv_producer_kernel<256>, a, gx) : cudaLaunchKernelEx(&cfg, kv_producer_kernel<512>, a, gx);

@@ -282,7 +282,7 @@ def attn_last_launch() -> tuple[int, int, int]:
 
 
 def attn_kernel_choice(args: AttnArgs) -> int:
-    """1 when `attn_fused` would run the tcgen05 kernel for these arguments, 0 for the mma.sync kernel."""
+    """What `attn_fused` would run for these arguments: 2 the prefill kernel, 1 the tcgen05 decode kernel, 0 mma.sync."""
     n = _lib.lib().nomos_attn_kernel_choice(C.byref(args))
     if n < 0:
         _check(int(n))

@@ -1,7 +1,7 @@
 """GPU parity of the prefill attention (many query rows, causal + sliding-window masks, no S x key_len scratch).
 
-int8 caches at head_dim 128 run on the query-major tcgen05 kernel (128 query rows per CTA); int4 / block-32 caches,
-wider heads and wrapped rings run as row groups of the mma.sync kernel.  Both are checked against the oracle's fp64
+int8 caches at head_dim 128 run on the query-major tcgen05 kernel; int4 / block-32 caches, wider heads and wrapped rings
+where a cost model finds it the faster one, else as row groups of the mma.sync kernel.  Both are checked against the oracle's fp64
 attention over the same cache bytes, every query row against its own RMS (2e-3), through the fused entry point and
 through the reference's square / prefix operators (lib/attention_gpu_int8.mojo:804-887).
 """
