@@ -135,12 +135,15 @@ __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32) append_i4_kernel(AppendI4
 // Head dims 128 / 256 / 512 without an int8 view: a warp per (token, KV head, K or V) row, held in registers and read once.
 // Launched with programmatic stream serialization on both sides: a decode step's append is a few KB between two attention
 // grids, whose set-up and settled tiles then overlap it (rows written here are newer than any the next grid may read early).
+// Longer appends hold the next grid back: their older rows are not among the newest few that it leaves for last, and there is
+// little to gain behind a chunk of a prompt.
 // Append + attention, 32q/4kv x 512 block-32 at 32768 keys: 57.4 us with a plain launch, 43.3 so; 9 rows + verify 29.8 / 27.9.
+constexpr int STEP_ROWS = 32;         // most tokens of a decode or verify step
 template <int HD, int FMT>
 __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32) append_rows_kernel(AppendI4Args a) {
     constexpr int NE = HD / 32;
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (a.n_s <= STEP_ROWS) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const long w = (long)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
     if (w >= 2l * a.n_s * a.nkv) return;
     const int lane = threadIdx.x & 31;

@@ -211,3 +211,37 @@ def test_paged_append_then_paged_attention_loop(oracle):
             want = oracle.attn_exact(q[i, b][None], c.k, c.v, c.ks, c.vs, c.kv_fmt, nh, nkv, hd, hd, per * page, S=1, query_base_pos=n, softmax_scale=0.1)
             ok, rel = within(got[i, b][None], want, TOL)
             assert ok, f"step {i} sequence {b}: {rel:.2e} x RMS"
+
+
+@pytest.mark.parametrize("fmt,hd,nh,nkv,path", [("i8", 128, 8, 4, "mma_sync"), ("i8", 128, 8, 4, "tcgen05"), ("i4b32", 512, 8, 2, "auto")])
+def test_a_long_append_holds_the_next_grid_back(oracle, fmt, hd, nh, nkv, path):
+    """A chunk of 400 rows, then one query row that declares all but the newest two settled: the chunk's rows are there, not
+    the ones that were in the cache before."""
+    rng = np.random.default_rng(191 + hd)
+    rounds, n_s = 6, 400
+    c = KVCache(fmt, nkv, n_s, hd)
+    ck, cv, cks, cvs = dev(c.k), dev(c.v), dev(c.ks), dev(c.vs)
+    q = bf16_normal(rng, (rounds, 1, nh, hd))
+    nk, nv = bf16_normal(rng, (rounds, n_s, nkv, hd)), bf16_normal(rng, (rounds, n_s, nkv, hd))
+    dq, dnk, dnv = dev(q), dev(nk), dev(nv)
+    outs = torch.full((rounds, 1, nh, hd), -1e30, dtype=torch.float32, device=DEV)
+    args = [ops.make_args(q=dq[i], k_cache=ck, v_cache=cv, k_scales=cks, v_scales=cvs, out=outs[i], kv_fmt=c.kv_fmt, S=1, nh=nh, nkv=nkv, kvg=nh // nkv, l_hd=hd,
+                          cache_hd=hd, cache_cap=n_s, klen=n_s, softmax_scale=0.1, flags=PATHS[path] | ops.SETTLED_CACHE) for i in range(rounds)]
+    need = max(ops.attn_workspace_bytes(a) for a in args)
+    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    for i, a in enumerate(args):
+        a.workspace, a.ws_bytes = ws.data_ptr(), need
+        rows = (dnk[i], dnv[i], ck, cv, cks, cvs, n_s, nkv, hd, nkv * hd, n_s, hd, 0)
+        if fmt == "i8":
+            ops.gpu_append_quant_kv_i8(None, *rows)
+        else:
+            ops.gpu_append_quant_kv_i4(None, *rows, c.scale_blocks)
+        ops.attn_fused(None, a)
+    torch.cuda.synchronize()
+    got = host(outs)
+    for i in range(rounds):
+        c.append(nk[i], nv[i], 0)
+        want = oracle.attn_exact(q[i], c.k, c.v, c.ks, c.vs, c.kv_fmt, nh, nkv, hd, hd, n_s, S=1, query_base_pos=n_s - 1, softmax_scale=0.1)
+        ok, rel = within(got[i], want, TOL)
+        assert ok, f"round {i}: {rel:.2e} x RMS"
